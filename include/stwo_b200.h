@@ -189,7 +189,8 @@ int stwo_precompute_twiddles(uint32_t root_initial_index, uint32_t root_step_siz
 /* In-place circle FFTs over columns of mixed sizes; column i has 2^log_sizes[i]
  * elements and its domain's half coset is a doubling of the tree's root coset.
  * Inverse FFTs include the 2^-log rescale.
- * Up to 64 columns travel in the launch parameters. Beyond that, these three
+ * Up to 64 columns travel in the launch parameters, and so does any number of columns
+ * of one size at equal distances (the rows of a matrix). Beyond that, these three
  * calls copy the column table into a pool buffer with a stream-ordered copy from
  * pageable host memory. Such a call may not be recorded into a CUDA graph; the
  * prover's own calls pass a prebuilt device table and stay graph-capturable. */

@@ -25,10 +25,11 @@
 //  * Zero extension for evaluate is fused into the first pass (the upper layers
 //    of a zero-padded input only copy it), the 2^-N rescale into the last pass.
 //  * One launch serves every column of one size: up to 64 columns travel by value
-//    in the parameter block; above that a device table of (src, dst) pointers
-//    (staged by the call, or resident in the caller's device memory) serves them
-//    all, so 2^16 columns take one launch per pass instead of 1024. Columns of
-//    different sizes use separate launches on the same stream.
+//    in the parameter block; above that columns at equal distances (a matrix's rows)
+//    travel as a base and a step, and others through a device table of (src, dst)
+//    pointers (staged by the call, or resident in the caller's device memory), so 2^16
+//    columns take one launch per pass instead of 1024. Columns of different sizes use
+//    separate launches on the same stream.
 #include <algorithm>
 #include <cstdlib>
 #include <utility>
@@ -52,6 +53,8 @@ struct FftLaunch {
     FftColumn cols[MAX_COLS_PER_LAUNCH];
     const FftColumn *table;  // device (src, dst) of every column, or null: cols[] above
     uint32_t src_from_dst;   // with a table: this pass reads table[col].dst (passes after the first)
+    uint32_t equidistant;    // column i at cols[0] + i * (src_step, dst_step) words
+    uint32_t src_step, dst_step;
     const uint32_t *tw;   // suffix of the tree for a size-2^N domain (2^(N-1) entries)
     uint32_t N;           // log size of the (virtual) transform
     uint32_t lo, hi;      // layers [lo, hi) applied by this pass
@@ -65,6 +68,8 @@ __device__ __forceinline__ uint32_t swz(uint32_t j) { return j ^ (((j >> 5) ^ (j
 
 // Source and destination of column `col` of a launch.
 __device__ __forceinline__ FftColumn fft_col(const FftLaunch &p, uint32_t col) {
+    if (p.equidistant)
+        return FftColumn{p.cols[0].src + (uint64_t)col * p.src_step, p.cols[0].dst + (uint64_t)col * p.dst_step};
     if (p.table) {
         const ulonglong2 t = __ldg(reinterpret_cast<const ulonglong2 *>(p.table) + col);
         FftColumn c{reinterpret_cast<const uint32_t *>(p.src_from_dst ? t.y : t.x), reinterpret_cast<uint32_t *>(t.y)};
@@ -221,14 +226,22 @@ __global__ void __launch_bounds__(1 << MAX_THREADS_LOG) fft_pass_kernel(const __
 // butterflies (the transform is bound by integer issue, not by HBM).
 //
 // Tile index bits: [0, C) columns of a strided tile (consecutive global words),
-// [C, C+G) the G layer bits of the pass, [C+G, 14) "slots": for a single-pass
-// transform of a 2^G column (G < 14) a CTA holds 2^(14-G) independent tiles.
+// [C, C+G) the G layer bits of the pass. A contiguous pass (C = 0) of G < 14 layers
+// holds 2^(14-G) independent groups: of one column, or of the several columns a tile of
+// short transforms covers (columns past the launch's last are neither read nor written).
 // The round structure is compile-time: the first round loads straight from global
 // memory into registers, the last round stores straight back, and only the rounds
 // in between go through shared memory, where the swizzled address is one XOR with
 // a constant (S is linear over GF(2); a round's own bits are disjoint from the
 // others). Middle rounds map warp lanes onto 5 tile bits whose bank images under
 // S are independent, so every shared-memory access is conflict free.
+// A strided pass right above the bottom one (its lowest layer is 14, every pass of
+// transforms up to 2^24) is compiled for that layer: its rows then lie at constant
+// distances and the loads and stores take them as immediate offsets. Measured with the
+// whole-line rows of turn_slot and the signed circle layer below (B200, us, before ->
+// after; interpolate, evaluate at blowup 2, at 4 for the first two): 8 x 2^24 754 -> 684,
+// 2756 -> 2423; 8 x 2^22 198 -> 173, 683 -> 577; 256 x 2^20 1260 -> 1101, 2381 -> 2014;
+// 101 x 2^16 50 -> 40, 78 -> 67.
 // CTA order: contiguous passes run the same tile position of all columns back to
 // back (their twiddles are then L2 hits); strided passes run the 2^(N-hi) copies of
 // an extension read back to back (the coefficient tile is then an L2 hit).
@@ -295,27 +308,47 @@ __device__ __forceinline__ uint32_t deposit(uint32_t x, const BitMap &m) {
     return r;
 }
 
+// Where a CTA's tile lies. Contiguous passes (C = 0): a tile is 2^14 consecutive
+// elements of one column, or all of 2^(14-N) columns of a shorter transform; it holds
+// 2^(14-G) independent groups of the pass's 2^G elements.
 struct GeoT {
     const FftLaunch *p;
-    uint32_t tiles_log, low_fixed, n_high, n_cols;
+    uint32_t n_cols;
+    uint32_t col;   // the tile's (first) column
+    uint32_t nc;    // log2 of a column's elements in the tile
+    uint32_t gfix;  // the tile's fixed global index bits
+    const uint32_t *src;
+    uint32_t *dst;  // of column col
 };
 
-template <int G, int C>
-__device__ __forceinline__ void tile_locate(const GeoT &geo, uint32_t jb, uint32_t &col, uint32_t &gidx) {
-    constexpr int SLOT_BITS = TT - C - G;
-    const uint32_t tile_id = (blockIdx.x << SLOT_BITS) | (jb >> (C + G));
-    const uint32_t jl = jb & ((1u << (C + G)) - 1u);
+// Global index of tile element jb within its column.
+template <int G, int C, int LO>
+__device__ __forceinline__ uint32_t tile_index(const GeoT &geo, uint32_t jb) {
     if constexpr (C == 0) {
-        // contiguous pass: tile position major, column minor
-        const uint32_t T = tile_id / geo.n_cols;
-        col = tile_id - T * geo.n_cols;
-        gidx = (T << G) | jl;
+        if constexpr (G == TT) return geo.gfix | jb;
+        else return geo.gfix | (jb & ((1u << geo.nc) - 1u));
     } else {
-        col = tile_id >> geo.tiles_log;
-        const uint32_t t = tile_id & ((1u << geo.tiles_log) - 1u);
-        const uint32_t th = t & ((1u << geo.n_high) - 1u), tl = t >> geo.n_high;
-        gidx = (tl << C) | (th << geo.p->hi) | (jl & ((1u << C) - 1u)) | ((jl >> C) << geo.p->lo);
+        const uint32_t lo = LO ? (uint32_t)LO : geo.p->lo;
+        return geo.gfix | (jb & ((1u << C) - 1u)) | ((jb >> C) << lo);
     }
+}
+
+// Source and destination of the column that tile element jb belongs to; false when the
+// launch has no such column (the last tile of a launch of short columns).
+template <int G, int C>
+__device__ __forceinline__ bool tile_column(const GeoT &geo, uint32_t jb, const uint32_t *&src, uint32_t *&dst) {
+    src = geo.src;
+    dst = geo.dst;
+    if constexpr (C == 0 && G < TT) {
+        if (geo.nc < (uint32_t)TT) {
+            const uint32_t col = geo.col + (jb >> geo.nc);
+            if (col >= geo.n_cols) return false;
+            const FftColumn fc = fft_col(*geo.p, col);
+            src = fc.src;
+            dst = fc.dst;
+        }
+    }
+    return true;
 }
 
 // The butterflies of one layer (bit u of the round) on one group of 2^RB registers.
@@ -327,11 +360,43 @@ __device__ __forceinline__ void layer_butterflies(uint32_t (&v)[1 << RB], const 
     constexpr bool CIRCLE = (C == 0 && A + U == 0);
     const uint32_t k = sh + U;
     const uint32_t hb = gb >> (k + 1);
-    uint32_t tws[NQ];
     if constexpr (CIRCLE) {
+        // Four butterflies share the first line layer's pair [x, y] as [y, -y, -x, x]; a
+        // negated twiddle only exchanges the butterfly's two outputs (or differences).
+        static_assert(NQ % 4 == 0, "the circle layer works on whole [x, y] pairs");
+        uint32_t xy[NQ / 2];
+        const uint32_t *tk = p.tw + (hb >> 1);
+        if constexpr (NQ >= 8) {
 #pragma unroll
-        for (int q = 0; q < NQ; q++) tws[q] = twiddle2(p.tw, p.N, 0, hb + q);
+            for (int q = 0; q < NQ / 2; q += 4) {
+                const uint4 t = __ldg(reinterpret_cast<const uint4 *>(tk + q));
+                xy[q] = t.x << 1; xy[q + 1] = t.y << 1; xy[q + 2] = t.z << 1; xy[q + 3] = t.w << 1;
+            }
+        } else {
+            const uint2 t = __ldg(reinterpret_cast<const uint2 *>(tk));
+            xy[0] = t.x << 1;
+            xy[1] = t.y << 1;
+        }
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+            const uint32_t t2 = xy[2 * (q >> 2) + (((q & 3) >> 1) ^ 1)];
+            uint32_t &a = v[2 * q], &b = v[2 * q + 1];
+            if ((q & 3) == 1 || (q & 3) == 2) {
+                if (INV) {
+                    const uint32_t s = m31_add(a, b), d = m31_sub(b, a);
+                    a = s;
+                    b = m31_mul2(d, t2);
+                } else {
+                    const uint32_t t = m31_mul2(b, t2);
+                    b = m31_add(a, t);
+                    a = m31_sub(a, t);
+                }
+            } else {
+                butterfly<INV>(a, b, t2);
+            }
+        }
     } else {
+        uint32_t tws[NQ];
         const uint32_t *tk = p.tw + ((1u << (p.N - 1)) - (1u << (p.N - k))) + hb;
         if constexpr (NQ >= 4) {
 #pragma unroll
@@ -346,13 +411,13 @@ __device__ __forceinline__ void layer_butterflies(uint32_t (&v)[1 << RB], const 
         } else {
             tws[0] = __ldg(tk) << 1;
         }
-    }
 #pragma unroll
-    for (int q = 0; q < NQ; q++) {
+        for (int q = 0; q < NQ; q++) {
 #pragma unroll
-        for (int l = 0; l < (1 << U); l++) {
-            const int m0 = (q << (U + 1)) | l;
-            butterfly<INV>(v[m0], v[m0 | (1 << U)], tws[q]);
+            for (int l = 0; l < (1 << U); l++) {
+                const int m0 = (q << (U + 1)) | l;
+                butterfly<INV>(v[m0], v[m0 | (1 << U)], tws[q]);
+            }
         }
     }
 }
@@ -372,93 +437,151 @@ __device__ __forceinline__ void round_butterflies(uint32_t (&v)[1 << RB], const 
     round_butterflies_seq<C, A, RB, INV>(v, p, gb, sh, std::make_integer_sequence<int, RB>{});
 }
 
-template <int C, int A, int RB, bool INV>
-__device__ __forceinline__ void store_global(uint32_t (&v)[1 << RB], const FftLaunch &p, uint32_t *__restrict__ dst,
-                                             uint32_t gb, uint32_t sh) {
-    constexpr int RR = 1 << RB;
-    if (INV && p.scale2) {
-#pragma unroll
-        for (int m = 0; m < RR; m++) v[m] = m31_mul2(v[m], p.scale2);
-    }
-    if constexpr (C == 0 && A == 0 && RR >= 4) {
-#pragma unroll
-        for (int m = 0; m < RR; m += 4)
-            *reinterpret_cast<uint4 *>(dst + gb + m) = make_uint4(v[m], v[m + 1], v[m + 2], v[m + 3]);
-    } else {
-#pragma unroll
-        for (int m = 0; m < RR; m++) dst[gb + ((uint32_t)m << sh)] = v[m];
-    }
+// A round that owns tile bits [0, RB) holds 2^RB consecutive elements in each thread. Read
+// or written directly, a warp's 16-byte accesses would each fall into 32 different lines
+// and half sectors; instead the warp moves its 2^(RB+5) consecutive elements as whole
+// lines and turns them in its own part of the shared tile. Row r of 2^RB words is thread
+// r's; its 16-byte chunk c lies in slot c ^ turn(r), so eight neighbouring lanes touch
+// eight different bank groups whether they read along a row or down a column of chunks.
+template <int RB>
+__device__ __forceinline__ uint32_t turn_slot(uint32_t r, uint32_t c) {
+    constexpr int LCH = RB - 2;
+    constexpr uint32_t CH = 1u << LCH;
+    const uint32_t f = LCH >= 3 ? (r & 7u) : ((r >> (3 - LCH)) & (CH - 1u));
+    return (r << LCH) + (c ^ f);
 }
 
-template <int G, int C, bool INV, int R, int E>
+template <int G, int C, bool INV, int R, int E, int LO>
 __device__ __forceinline__ void roundT(uint32_t *sm, const GeoT &geo) {
     using RI = RoundT<G, INV, R, E>;
     constexpr int RB = RI::RB, A = RI::A, OA = C + A, RR = 1 << RB, GROUPS = 1 << (E - RB), W = TT - E;
     constexpr bool FIRST = R == 0, LAST = R == RI::NR - 1;
+    constexpr bool ROWS = C == 0 && A == 0;  // a thread's elements are consecutive
+    constexpr int CH = ROWS ? RR / 4 : 1;    // its 16-byte chunks
     constexpr int XBITS = TT - RB;
     constexpr BitMap M = make_map(OA, RB, !FIRST && !LAST);
     const FftLaunch &p = *geo.p;
-    const uint32_t lo = (C == 0) ? 0u : p.lo;
+    const uint32_t lo = (C == 0) ? 0u : LO ? (uint32_t)LO : p.lo;
     const uint32_t sh = lo + A;  // global bit of the round's first owned bit
     const uint32_t jt = deposit<W>(threadIdx.x, M);
+    const uint32_t lane = threadIdx.x & 31u;
+    uint4 *sm4 = reinterpret_cast<uint4 *>(sm);
+
+    uint32_t v[FIRST ? GROUPS : 1][RR];
     if constexpr (FIRST) {
         // Issue every global load of the round before the first butterfly.
-        uint32_t v[GROUPS][RR];
-        uint32_t gbs[GROUPS], cols[GROUPS];
 #pragma unroll
         for (int grp = 0; grp < GROUPS; grp++) {
             const uint32_t jb = jt | deposit<XBITS>((uint32_t)grp << W, M);
-            tile_locate<G, C>(geo, jb, cols[grp], gbs[grp]);
-            const uint32_t *__restrict__ src = fft_col(p, cols[grp]).src;
-            const uint32_t base = gbs[grp] & p.src_mask;
-            if constexpr (C == 0 && A == 0 && RR >= 4) {
+            if constexpr (ROWS) {
+                const uint32_t region = jb & ~((32u << RB) - 1u);
+                // (a warp's part within one column, the usual case: its base once)
+                const uint32_t *src;
+                uint32_t *dst;
+                const bool whole = G >= RB + 5 || geo.nc >= (uint32_t)(RB + 5);
+                const bool there = tile_column<G, C>(geo, region, src, dst);
+                src += (tile_index<G, C, LO>(geo, region) & p.src_mask) + 4u * lane;
 #pragma unroll
-                for (int m = 0; m < RR; m += 4) {
-                    uint4 t = __ldg(reinterpret_cast<const uint4 *>(src + base + m));
-                    v[grp][m] = t.x; v[grp][m + 1] = t.y; v[grp][m + 2] = t.z; v[grp][m + 3] = t.w;
+                for (int i = 0; i < CH; i++) {
+                    uint4 t = make_uint4(0, 0, 0, 0);
+                    if (whole && (G >= RB + 5 || p.src_mask >= (32u << RB) - 1u)) {
+                        if (there) t = __ldg(reinterpret_cast<const uint4 *>(src + 128u * i));
+                    } else {
+                        const uint32_t e = region + 4u * (i * 32u + lane);
+                        const uint32_t *s2;
+                        if (tile_column<G, C>(geo, e, s2, dst))
+                            t = __ldg(reinterpret_cast<const uint4 *>(s2 + (tile_index<G, C, LO>(geo, e) & p.src_mask)));
+                    }
+                    v[grp][4 * i] = t.x; v[grp][4 * i + 1] = t.y; v[grp][4 * i + 2] = t.z; v[grp][4 * i + 3] = t.w;
                 }
             } else {
+                const uint32_t *src;
+                uint32_t *dst;
+                const bool there = tile_column<G, C>(geo, jb, src, dst);
+                src += tile_index<G, C, LO>(geo, jb) & p.src_mask;
 #pragma unroll
-                for (int m = 0; m < RR; m++) v[grp][m] = __ldg(src + base + ((uint32_t)m << sh));
-            }
-        }
-#pragma unroll
-        for (int grp = 0; grp < GROUPS; grp++) {
-            round_butterflies<C, A, RB, INV>(v[grp], p, gbs[grp], sh);
-            if constexpr (LAST) {
-                store_global<C, A, RB, INV>(v[grp], p, fft_col(p, cols[grp]).dst, gbs[grp], sh);
-            } else {
-                const uint32_t sj = swz_c(jt | deposit<XBITS>((uint32_t)grp << W, M));
-#pragma unroll
-                for (int m = 0; m < RR; m++) sm[sj ^ swz_c((uint32_t)m << OA)] = v[grp][m];
-            }
-        }
-    } else {
-#pragma unroll 1
-        for (int grp = 0; grp < GROUPS; grp++) {
-            const uint32_t jb = jt | deposit<XBITS>((uint32_t)grp << W, M);
-            uint32_t col, gb;
-            tile_locate<G, C>(geo, jb, col, gb);
-            uint32_t v[RR];
-            const uint32_t sj = swz_c(jb);
-#pragma unroll
-            for (int m = 0; m < RR; m++) v[m] = sm[sj ^ swz_c((uint32_t)m << OA)];
-            round_butterflies<C, A, RB, INV>(v, p, gb, sh);
-            if constexpr (LAST) {
-                store_global<C, A, RB, INV>(v, p, fft_col(p, col).dst, gb, sh);
-            } else {
-#pragma unroll
-                for (int m = 0; m < RR; m++) sm[sj ^ swz_c((uint32_t)m << OA)] = v[m];
+                for (int m = 0; m < RR; m++) v[grp][m] = there ? __ldg(src + ((size_t)m << sh)) : 0u;
             }
         }
     }
+    auto group = [&](int grp, uint32_t (&w)[RR]) {
+        const uint32_t jb = jt | deposit<XBITS>((uint32_t)grp << W, M);
+        const uint32_t gb = tile_index<G, C, LO>(geo, jb);
+        const uint32_t region = jb & ~((32u << RB) - 1u);
+        const uint32_t sj = swz_c(jb);
+        if constexpr (FIRST && ROWS) {
+#pragma unroll
+            for (int i = 0; i < CH; i++) {
+                const uint32_t q = i * 32u + lane;
+                sm4[(region >> 2) + turn_slot<RB>(q / CH, q % CH)] =
+                    make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < CH; c++) {
+                const uint4 t = sm4[(region >> 2) + turn_slot<RB>(lane, c)];
+                w[4 * c] = t.x; w[4 * c + 1] = t.y; w[4 * c + 2] = t.z; w[4 * c + 3] = t.w;
+            }
+            __syncwarp();
+        }
+        if constexpr (!FIRST) {
+#pragma unroll
+            for (int m = 0; m < RR; m++) w[m] = sm[sj ^ swz_c((uint32_t)m << OA)];
+        }
+        round_butterflies<C, A, RB, INV>(w, p, gb, sh);
+        if constexpr (!LAST) {
+#pragma unroll
+            for (int m = 0; m < RR; m++) sm[sj ^ swz_c((uint32_t)m << OA)] = w[m];
+        } else {
+            if (INV && p.scale2) {
+#pragma unroll
+                for (int m = 0; m < RR; m++) w[m] = m31_mul2(w[m], p.scale2);
+            }
+            const uint32_t *src;
+            uint32_t *dst;
+            if constexpr (ROWS) {
+                __syncwarp();
+#pragma unroll
+                for (int c = 0; c < CH; c++)
+                    sm4[(region >> 2) + turn_slot<RB>(lane, c)] =
+                        make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+                __syncwarp();
+                const bool whole = G >= RB + 5 || geo.nc >= (uint32_t)(RB + 5);
+                const bool there = tile_column<G, C>(geo, region, src, dst);
+                dst += tile_index<G, C, LO>(geo, region) + 4u * lane;
+#pragma unroll
+                for (int i = 0; i < CH; i++) {
+                    const uint32_t q = i * 32u + lane, e = region + 4u * q;
+                    const uint4 t = sm4[(region >> 2) + turn_slot<RB>(q / CH, q % CH)];
+                    if (whole) {
+                        if (there) *reinterpret_cast<uint4 *>(dst + 128u * i) = t;
+                    } else {
+                        uint32_t *d2;
+                        if (tile_column<G, C>(geo, e, src, d2))
+                            *reinterpret_cast<uint4 *>(d2 + tile_index<G, C, LO>(geo, e)) = t;
+                    }
+                }
+            } else if (tile_column<G, C>(geo, jb, src, dst)) {
+                dst += gb;
+#pragma unroll
+                for (int m = 0; m < RR; m++) dst[(size_t)m << sh] = w[m];
+            }
+        }
+    };
+    if constexpr (FIRST) {
+#pragma unroll
+        for (int grp = 0; grp < GROUPS; grp++) group(grp, v[grp]);
+    } else {
+#pragma unroll 1
+        for (int grp = 0; grp < GROUPS; grp++) group(grp, v[0]);
+    }
 }
 
-template <int G, int C, bool INV, int E, int... Rs>
+template <int G, int C, bool INV, int E, int LO, int... Rs>
 __device__ __forceinline__ void roundsT(uint32_t *sm, const GeoT &geo, std::integer_sequence<int, Rs...>) {
     (
         [&] {
-            roundT<G, C, INV, Rs, E>(sm, geo);
+            roundT<G, C, INV, Rs, E, LO>(sm, geo);
             if constexpr (Rs + 1 < RoundT<G, INV, 0, E>::NR) __syncthreads();
         }(),
         ...);
@@ -468,23 +591,40 @@ __device__ __forceinline__ void roundsT(uint32_t *sm, const GeoT &geo, std::inte
 // shared memory), measured 2292 vs 2231 columns/s at log 24 against two CTAs per SM
 // with 112-128 registers, and 2132 with four CTAs per SM (64 registers). 2^5 elements
 // a thread (512 threads): two CTAs per SM (64 registers; at three it spills).
-template <int G, int C, bool INV, int E>
+template <int G, int C, bool INV, int E, int LO>
 __global__ void __launch_bounds__(1 << (TT - E), E == 6 ? 3 : 2) fftT_kernel(const __grid_constant__ FftLaunch p, uint32_t n_cols) {
-    extern __shared__ uint32_t sm[];
+    extern __shared__ __align__(16) uint32_t sm[];
     GeoT geo;
     geo.p = &p;
-    geo.tiles_log = p.N - (C + G);
-    geo.low_fixed = (C == 0) ? 0u : p.lo - C;
-    geo.n_high = p.N - p.hi;
     geo.n_cols = n_cols;
-    roundsT<G, C, INV, E>(sm, geo, std::make_integer_sequence<int, RoundT<G, INV, 0, E>::NR>{});
+    geo.nc = min(p.N, (uint32_t)TT);
+    if constexpr (C == 0) {
+        if (G == TT || p.N >= (uint32_t)TT) {
+            // tile position major, column minor
+            const uint32_t T = blockIdx.x / n_cols;
+            geo.col = blockIdx.x - T * n_cols;
+            geo.gfix = T << TT;
+        } else {
+            geo.col = blockIdx.x << (TT - p.N);
+            geo.gfix = 0;
+        }
+    } else {
+        const uint32_t tiles_log = p.N - (C + G), n_high = p.N - p.hi;
+        const uint32_t t = blockIdx.x & ((1u << tiles_log) - 1u);
+        geo.col = blockIdx.x >> tiles_log;
+        geo.gfix = ((t >> n_high) << C) | ((t & ((1u << n_high) - 1u)) << p.hi);
+    }
+    const FftColumn fc = fft_col(p, geo.col);
+    geo.src = fc.src;
+    geo.dst = fc.dst;
+    roundsT<G, C, INV, E, LO>(sm, geo, std::make_integer_sequence<int, RoundT<G, INV, 0, E>::NR>{});
 }
 
-template <int G, int C, bool INV, int E>
+template <int G, int C, bool INV, int E, int LO>
 int launchT_e(const FftLaunch &p, uint32_t n_cols, cudaStream_t st) {
     constexpr int NR = RoundT<G, INV, 0, E>::NR;
-    const size_t smem = NR > 1 ? (sizeof(uint32_t) << TT) : 0;
-    auto kern = fftT_kernel<G, C, INV, E>;
+    const size_t smem = NR > 1 || C == 0 ? (sizeof(uint32_t) << TT) : 0;
+    auto kern = fftT_kernel<G, C, INV, E, LO>;
     static std::atomic<uint64_t> attr_set{0};
     int rc = once_per_device(attr_set, [&] {
         STWO_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -492,11 +632,9 @@ int launchT_e(const FftLaunch &p, uint32_t n_cols, cudaStream_t st) {
         return (int)STWO_OK;
     });
     if (rc) return rc;
-    const uint64_t tiles = (uint64_t)n_cols << (p.N - C - G);
-    const uint64_t per_cta = 1ull << (TT - C - G);
-    STWO_REQUIRE(tiles % per_cta == 0, STWO_ERR_UNSUPPORTED_SIZE, "fft tile packing");
-    STWO_REQUIRE(tiles < (1ull << 32), STWO_ERR_UNSUPPORTED_SIZE, "fft launch of %llu tiles", (unsigned long long)tiles);
-    const uint64_t blocks = tiles / per_cta;
+    const uint64_t blocks = p.N >= (uint32_t)TT ? (uint64_t)n_cols << (p.N - TT)
+                                                : ((uint64_t)n_cols + (1u << (TT - p.N)) - 1) >> (TT - p.N);
+    STWO_REQUIRE(blocks < (1ull << 31), STWO_ERR_UNSUPPORTED_SIZE, "fft launch of %llu tiles", (unsigned long long)blocks);
     kern<<<(unsigned)blocks, 1 << (TT - E), smem, st>>>(p, n_cols);
     STWO_LAUNCH_CHECK("fftT_kernel");
     return STWO_OK;
@@ -514,17 +652,26 @@ inline int fft_ept_log(bool contiguous, uint32_t N) {
     return tunable(!contiguous ? TUNE_FFT_EPT_STRIDED : N <= 20 ? TUNE_FFT_EPT_CONTIG_SMALL : TUNE_FFT_EPT_CONTIG_LARGE);
 }
 
-template <int G, int C, bool INV>
+template <int G, int C, bool INV, int LO = 0>
 int launchT_t(const FftLaunch &p, uint32_t n_cols, cudaStream_t st) {
-    return fft_ept_log(C == 0, p.N) == 5 ? launchT_e<G, C, INV, 5>(p, n_cols, st) : launchT_e<G, C, INV, 6>(p, n_cols, st);
+    if constexpr (C > 0 || G >= 11)
+        if (fft_ept_log(C == 0, p.N) == 5) return launchT_e<G, C, INV, 5, 0>(p, n_cols, st);
+    return launchT_e<G, C, INV, 6, LO>(p, n_cols, st);
 }
 
-// Dispatch over (G, C): contiguous passes G = 11..14 (C = 0), strided passes
+// Dispatch over (G, C): contiguous passes G = 4..14 (C = 0), strided passes
 // G = 1..10 with C = 14 - G.
 template <bool INV>
 int launchT(const FftLaunch &p, uint32_t n_cols, uint32_t G, uint32_t C, cudaStream_t st) {
     if (C == 0) {
         switch (G) {
+        case 4: return launchT_t<4, 0, INV>(p, n_cols, st);
+        case 5: return launchT_t<5, 0, INV>(p, n_cols, st);
+        case 6: return launchT_t<6, 0, INV>(p, n_cols, st);
+        case 7: return launchT_t<7, 0, INV>(p, n_cols, st);
+        case 8: return launchT_t<8, 0, INV>(p, n_cols, st);
+        case 9: return launchT_t<9, 0, INV>(p, n_cols, st);
+        case 10: return launchT_t<10, 0, INV>(p, n_cols, st);
         case 11: return launchT_t<11, 0, INV>(p, n_cols, st);
         case 12: return launchT_t<12, 0, INV>(p, n_cols, st);
         case 13: return launchT_t<13, 0, INV>(p, n_cols, st);
@@ -532,17 +679,27 @@ int launchT(const FftLaunch &p, uint32_t n_cols, uint32_t G, uint32_t C, cudaStr
         default: break;
         }
     } else if (C + G == TT) {
+        if (p.lo == (uint32_t)TT) {
+            switch (G) {
+            case 6: return launchT_t<6, TT - 6, INV, TT>(p, n_cols, st);
+            case 7: return launchT_t<7, TT - 7, INV, TT>(p, n_cols, st);
+            case 8: return launchT_t<8, TT - 8, INV, TT>(p, n_cols, st);
+            case 9: return launchT_t<9, TT - 9, INV, TT>(p, n_cols, st);
+            case 10: return launchT_t<10, TT - 10, INV, TT>(p, n_cols, st);
+            default: break;
+            }
+        }
         switch (G) {
-        case 1: return launchT_t<1, 13, INV>(p, n_cols, st);
-        case 2: return launchT_t<2, 12, INV>(p, n_cols, st);
-        case 3: return launchT_t<3, 11, INV>(p, n_cols, st);
-        case 4: return launchT_t<4, 10, INV>(p, n_cols, st);
-        case 5: return launchT_t<5, 9, INV>(p, n_cols, st);
-        case 6: return launchT_t<6, 8, INV>(p, n_cols, st);
-        case 7: return launchT_t<7, 7, INV>(p, n_cols, st);
-        case 8: return launchT_t<8, 6, INV>(p, n_cols, st);
-        case 9: return launchT_t<9, 5, INV>(p, n_cols, st);
-        case 10: return launchT_t<10, 4, INV>(p, n_cols, st);
+        case 1: return launchT_t<1, TT - 1, INV>(p, n_cols, st);
+        case 2: return launchT_t<2, TT - 2, INV>(p, n_cols, st);
+        case 3: return launchT_t<3, TT - 3, INV>(p, n_cols, st);
+        case 4: return launchT_t<4, TT - 4, INV>(p, n_cols, st);
+        case 5: return launchT_t<5, TT - 5, INV>(p, n_cols, st);
+        case 6: return launchT_t<6, TT - 6, INV>(p, n_cols, st);
+        case 7: return launchT_t<7, TT - 7, INV>(p, n_cols, st);
+        case 8: return launchT_t<8, TT - 8, INV>(p, n_cols, st);
+        case 9: return launchT_t<9, TT - 9, INV>(p, n_cols, st);
+        case 10: return launchT_t<10, TT - 10, INV>(p, n_cols, st);
         default: break;
         }
     }
@@ -772,11 +929,21 @@ int fft_columns_tab(const uint32_t *const *srcs, uint32_t *const *dsts, uint32_t
     FftLaunch p{};
     p.tw = tree + (tree_size - (1ull << (N - 1)));
     p.N = N;
-    // More than 64 columns: every pass is one launch over a device table.
+    // More than 64 columns: every pass is one launch, over columns at equal distances (the
+    // rows of one matrix) or over a device table.
     const FftColumn *table = nullptr;
     void *staged = nullptr;
     if (n_cols > (uint32_t)MAX_COLS_PER_LAUNCH) {
-        if (dev_table) {
+        const intptr_t src_step = (intptr_t)srcs[1] - (intptr_t)srcs[0], dst_step = (intptr_t)dsts[1] - (intptr_t)dsts[0];
+        bool equidistant = src_step > 0 && dst_step > 0 && src_step < (1ll << 34) && dst_step < (1ll << 34);
+        for (uint32_t i = 1; i < n_cols && equidistant; i++)
+            equidistant = (intptr_t)srcs[i] - (intptr_t)srcs[i - 1] == src_step &&
+                          (intptr_t)dsts[i] - (intptr_t)dsts[i - 1] == dst_step;
+        if (equidistant) {
+            p.equidistant = 1;
+            p.src_step = (uint32_t)(src_step / 4);
+            p.dst_step = (uint32_t)(dst_step / 4);
+        } else if (dev_table) {
             table = static_cast<const FftColumn *>(dev_table);
         } else {
             std::vector<FftColumn> h(n_cols);
@@ -806,22 +973,27 @@ int fft_columns_tab(const uint32_t *const *srcs, uint32_t *const *dsts, uint32_t
         bool first = pi == 0, last = pi + 1 == passes.size();
         p.src_mask = (first && L < N) ? ((1u << L) - 1u) : 0xffffffffu;
         p.scale2 = (inv && last) ? (m31_inv_pow2(N) << 1) : 0u;
-        const uint32_t per_launch = table ? n_cols : (uint32_t)MAX_COLS_PER_LAUNCH;
+        const uint32_t per_launch = table || p.equidistant ? n_cols : (uint32_t)MAX_COLS_PER_LAUNCH;
+        if (!first) p.src_step = p.dst_step;
         p.table = table;
         p.src_from_dst = first ? 0u : 1u;
         for (uint32_t base = 0; base < n_cols; base += per_launch) {
             uint32_t cnt = std::min<uint32_t>(per_launch, n_cols - base);
             if (!table)
-                for (uint32_t i = 0; i < cnt; i++)
+                for (uint32_t i = 0; i < std::min<uint32_t>(cnt, MAX_COLS_PER_LAUNCH); i++)
                     p.cols[i] = FftColumn{first ? srcs[base + i] : dsts[base + i], dsts[base + i]};
             const uint32_t G = ps.hi - ps.lo;
-            // Specialised 2^15 tiles: strided passes, or contiguous passes of >= 11 layers whose
-            // tiles pack evenly into CTAs.
+            // Tiles of 2^14 elements: strided passes, and contiguous passes of 4 layers or more.
+            // A launch of short columns with fewer elements than this fills too few SMs with
+            // them, and one CTA a column (launch_pass) is faster: us of interpolate / evaluate
+            // at blowup 2, tiles against CTAs of a column: 512 x 2^10 13.3 / 13.3 and
+            // 11.4 / 15.4, 2048 x 2^8 15.3 / 13.6 and 11.2 / 13.3, 32768 x 2^4 13.3 / 11.2 and
+            // 26 / 46, 65536 x 2^10 at blowup 4 165 / 550 and 598 / 2218.
             // (vector twiddle loads need the tree suffix 16-byte aligned)
+            const bool fills = G >= 11 || ((uint64_t)cnt << N) >= (G > 5 ? 1ull << 20 : 1ull << 18);
             const bool spec = ((uintptr_t)p.tw & 15) == 0 &&
                               ((ps.c > 0 && ps.tile_log == (uint32_t)TT) ||
-                               (ps.c == 0 && G >= 11 && G <= (uint32_t)TT &&
-                                ((uint64_t)cnt << (N - G)) % (1ull << (TT - G)) == 0));
+                               (ps.c == 0 && G >= 4 && G <= (uint32_t)TT && fills));
             int rc = spec ? (inv ? launchT<true>(p, cnt, G, ps.c, st) : launchT<false>(p, cnt, G, ps.c, st))
                           : launch_pass(p, cnt, inv, st);
             if (rc) return rc;

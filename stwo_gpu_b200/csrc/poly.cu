@@ -464,8 +464,17 @@ uint32_t eval_at_point_blocks(uint32_t log_size, uint32_t iter_log) {
 
 uint32_t eval_at_point_iter_log(const uint32_t *log_sizes, uint32_t n) { return eap_iter_log(log_sizes, n); }
 
+// Whether all n columns have one size: they are then one launch sequence as they are.
+static bool same_size(const uint32_t *logs, uint32_t n) {
+    for (uint32_t i = 1; i < n; i++)
+        if (logs[i] != logs[0]) return false;
+    return true;
+}
+
 int extend_evaluate_async(const uint32_t *const *coeffs, const uint32_t *coeff_logs, uint32_t *const *outs,
                           uint32_t log_blowup, uint32_t n, const uint32_t *tw, uint64_t tree_size, cudaStream_t st) {
+    if (n && log_blowup && coeff_logs[0] + log_blowup > 2 && same_size(coeff_logs, n))
+        return fft_columns(coeffs, outs, n, coeff_logs[0] + log_blowup, coeff_logs[0], tw, tree_size, false, st);
     // Group columns by size so each size is one launch sequence.
     std::map<uint32_t, std::vector<uint32_t>> by_size;
     for (uint32_t i = 0; i < n; i++) by_size[coeff_logs[i]].push_back(i);
@@ -495,6 +504,7 @@ int extend_evaluate_async(const uint32_t *const *coeffs, const uint32_t *coeff_l
 
 int columns_fft_async(uint32_t *const *cols, const uint32_t *logs, uint32_t n, const uint32_t *tree,
                       uint64_t tree_size, bool inv, cudaStream_t st) {
+    if (n && same_size(logs, n)) return fft_columns(cols, cols, n, logs[0], logs[0], tree, tree_size, inv, st);
     std::map<uint32_t, std::vector<uint32_t *>> by_size;
     for (uint32_t i = 0; i < n; i++) by_size[logs[i]].push_back(cols[i]);
     for (auto &kv : by_size) {
