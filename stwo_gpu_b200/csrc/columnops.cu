@@ -93,6 +93,7 @@ struct FieldT<uint32_t> {
 template <typename F>
 __global__ void __launch_bounds__(BI_THREADS) batch_inverse_kernel(const F *__restrict__ src, F *__restrict__ dst,
                                                                     uint64_t n) {
+    chain_wait();
     using T = FieldT<F>;
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t warp_global = ((uint64_t)blockIdx.x * BI_THREADS + threadIdx.x) >> 5;
@@ -138,6 +139,7 @@ __global__ void __launch_bounds__(BI_THREADS) batch_inverse_kernel(const F *__re
 // unique, so the values are the same.
 __global__ void __launch_bounds__(BI_THREADS) batch_inverse_qm31_norm_kernel(const qm31 *__restrict__ src,
                                                                              qm31 *__restrict__ dst, uint64_t n) {
+    chain_wait();
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t warp_global = ((uint64_t)blockIdx.x * BI_THREADS + threadIdx.x) >> 5;
     const uint64_t base = warp_global * (32 * BI_PER_THREAD) + lane;
@@ -235,7 +237,7 @@ int bit_reverse_async(uint32_t *col, uint64_t n, uint32_t words, cudaStream_t st
 int batch_inverse_m31_async(const uint32_t *src, uint32_t *dst, uint64_t n, cudaStream_t st) {
     if (n == 0) return STWO_OK;
     uint64_t blocks = (n + BI_THREADS * BI_PER_THREAD - 1) / (BI_THREADS * BI_PER_THREAD);
-    batch_inverse_kernel<uint32_t><<<(unsigned)blocks, BI_THREADS, 0, st>>>(src, dst, n);
+    launch_chained(batch_inverse_kernel<uint32_t>, (unsigned)blocks, BI_THREADS, 0, st, src, dst, n);
     STWO_LAUNCH_CHECK("batch_inverse_kernel<m31>");
     return STWO_OK;
 }
@@ -243,7 +245,7 @@ int batch_inverse_m31_async(const uint32_t *src, uint32_t *dst, uint64_t n, cuda
 int batch_inverse_qm31_async(const uint32_t *src, uint32_t *dst, uint64_t n, cudaStream_t st) {
     if (n == 0) return STWO_OK;
     uint64_t blocks = (n + BI_THREADS * BI_PER_THREAD - 1) / (BI_THREADS * BI_PER_THREAD);
-    batch_inverse_qm31_norm_kernel<<<(unsigned)blocks, BI_THREADS, 0, st>>>(reinterpret_cast<const qm31 *>(src),
+    launch_chained(batch_inverse_qm31_norm_kernel, (unsigned)blocks, BI_THREADS, 0, st, reinterpret_cast<const qm31 *>(src),
                                                                             reinterpret_cast<qm31 *>(dst), n);
     STWO_LAUNCH_CHECK("batch_inverse_qm31_norm_kernel");
     return STWO_OK;

@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <utility>
 
 #include "../../include/stwo_b200.h"
 #include "field.cuh"
@@ -47,6 +48,35 @@ inline void count_launch(uint64_t n = 1) {
     do {                                                                                  \
         if (!(cond)) return ::stwo::set_error(status, __VA_ARGS__);                       \
     } while (0)
+
+// Launches k so that its CTAs are placed as the CTAs of the kernel before it on the stream
+// exit, instead of after that kernel has completed and been flushed (programmatic dependent
+// launch). Every kernel launched this way calls chain_wait() before it touches memory: the
+// call returns once the kernel before has completed, all its writes visible. Since that
+// kernel waited for the one before it in turn, stream order holds throughout; a kernel or
+// copy enqueued the ordinary way before or after is waited for, or waits, as ever.
+// What it saves is the gap between short kernels, measured on the B200 (us, before ->
+// after): 20 folds of 2^24 values down to 2^4 225 -> 185, the four passes of 101 x 2^16
+// interpolate + evaluate 92.7 -> 83.5; a captured small proof 646 -> 639. Letting the next
+// kernel's CTAs in earlier (griddepcontrol.launch_dependents at the start of every kernel)
+// measured the same (186, 83.5, 650-658) and would let waiting CTAs hold SM slots.
+template <class... KArgs, class... Args>
+inline void launch_chained(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);  // (the caller's STWO_LAUNCH_CHECK reads its error)
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
 
 inline bool is_pow2(uint64_t n) { return n && !(n & (n - 1)); }
 inline uint32_t log2_u64(uint64_t n) {

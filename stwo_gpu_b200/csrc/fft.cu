@@ -162,6 +162,7 @@ __device__ __forceinline__ void fft_round_dispatch(int rb, uint32_t *sm, const F
 template <int LOG_E, bool INV>
 __global__ void __launch_bounds__(1 << MAX_THREADS_LOG) fft_pass_kernel(const __grid_constant__ FftLaunch p) {
     extern __shared__ uint32_t sm[];
+    chain_wait();
     const uint32_t tile = 1u << p.tile_log;
     const uint32_t W = p.tile_log - LOG_E;  // log2(threads)
     const uint32_t tiles_log = p.N - p.tile_log;
@@ -594,6 +595,7 @@ __device__ __forceinline__ void roundsT(uint32_t *sm, const GeoT &geo, std::inte
 template <int G, int C, bool INV, int E, int LO>
 __global__ void __launch_bounds__(1 << (TT - E), E == 6 ? 3 : 2) fftT_kernel(const __grid_constant__ FftLaunch p, uint32_t n_cols) {
     extern __shared__ __align__(16) uint32_t sm[];
+    chain_wait();
     GeoT geo;
     geo.p = &p;
     geo.n_cols = n_cols;
@@ -635,7 +637,7 @@ int launchT_e(const FftLaunch &p, uint32_t n_cols, cudaStream_t st) {
     const uint64_t blocks = p.N >= (uint32_t)TT ? (uint64_t)n_cols << (p.N - TT)
                                                 : ((uint64_t)n_cols + (1u << (TT - p.N)) - 1) >> (TT - p.N);
     STWO_REQUIRE(blocks < (1ull << 31), STWO_ERR_UNSUPPORTED_SIZE, "fft launch of %llu tiles", (unsigned long long)blocks);
-    kern<<<(unsigned)blocks, 1 << (TT - E), smem, st>>>(p, n_cols);
+    launch_chained(kern, (unsigned)blocks, 1 << (TT - E), smem, st, p, n_cols);
     STWO_LAUNCH_CHECK("fftT_kernel");
     return STWO_OK;
 }
@@ -764,7 +766,7 @@ int launch_pass_t(const FftLaunch &p, uint32_t n_cols, cudaStream_t st) {
     if (rc) return rc;
     const uint64_t blocks = (uint64_t)n_cols << (p.N - p.tile_log);
     STWO_REQUIRE(blocks < (1ull << 31), STWO_ERR_UNSUPPORTED_SIZE, "fft grid too large");
-    kern<<<(unsigned)blocks, threads, smem, st>>>(p);
+    launch_chained(kern, (unsigned)blocks, threads, smem, st, p);
     STWO_LAUNCH_CHECK("fft_pass_kernel");
     return STWO_OK;
 }

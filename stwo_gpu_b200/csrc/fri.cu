@@ -28,6 +28,7 @@ template <bool CIRCLE, bool JOBS>
 __global__ void fold_kernel(const __grid_constant__ Cols4 src_p, const __grid_constant__ MutCols4 dst_p, uint64_t n_out,
                             const uint32_t *__restrict__ tw, qm31 alpha, qm31 alpha_sq, const qm31 *alpha_dev,
                             size_t js) {
+    chain_wait();
     // the column pointers stay in the parameter block; a job's offset is added at each
     // use (a multiply-add) rather than holding eight moved pointers in registers
     const size_t jo = JOBS ? (size_t)blockIdx.y * js : 0;
@@ -97,6 +98,7 @@ template <bool CIRCLE>
 __global__ void fold_small_kernel(const __grid_constant__ Cols4 src_p, const __grid_constant__ MutCols4 dst_p,
                                   uint32_t n_out, uint32_t t0, uint32_t t1, const uint32_t *tw, qm31 alpha,
                                   qm31 alpha_sq, const qm31 *alpha_dev, size_t js) {
+    chain_wait();
     Cols4 src;
     MutCols4 dst;
     for (int c = 0; c < 4; c++) {
@@ -155,8 +157,8 @@ int fold_async(const uint32_t *const *src4, uint64_t n, stwo_qm31 alpha_c, const
             t[1] = m31_neg(iy);
         }
         if (circle)
-            fold_small_kernel<true><<<jobs, 1, 0, st>>>(s, d, (uint32_t)n_out, t[0], t[1], nullptr, alpha, a2, ad, js);
-        else fold_small_kernel<false><<<jobs, 1, 0, st>>>(s, d, (uint32_t)n_out, 0u, 0u, tw, alpha, a2, ad, js);
+            launch_chained(fold_small_kernel<true>, jobs, 1, 0, st, s, d, (uint32_t)n_out, t[0], t[1], (const uint32_t *)nullptr, alpha, a2, ad, js);
+        else launch_chained(fold_small_kernel<false>, jobs, 1, 0, st, s, d, (uint32_t)n_out, 0u, 0u, tw, alpha, a2, ad, js);
         STWO_LAUNCH_CHECK("fold_small_kernel");
         return STWO_OK;
     }
@@ -168,11 +170,11 @@ int fold_async(const uint32_t *const *src4, uint64_t n, stwo_qm31 alpha_c, const
     if (blocks > cap) blocks = cap;
     const dim3 grid(blocks, jobs);
     if (jobs > 1) {
-        if (circle) fold_kernel<true, true><<<grid, 256, 0, st>>>(s, d, n_out, tw, alpha, a2, ad, js);
-        else fold_kernel<false, true><<<grid, 256, 0, st>>>(s, d, n_out, tw, alpha, a2, ad, js);
+        if (circle) launch_chained(fold_kernel<true, true>, grid, 256, 0, st, s, d, n_out, tw, alpha, a2, ad, js);
+        else launch_chained(fold_kernel<false, true>, grid, 256, 0, st, s, d, n_out, tw, alpha, a2, ad, js);
     } else {
-        if (circle) fold_kernel<true, false><<<grid, 256, 0, st>>>(s, d, n_out, tw, alpha, a2, ad, 0);
-        else fold_kernel<false, false><<<grid, 256, 0, st>>>(s, d, n_out, tw, alpha, a2, ad, 0);
+        if (circle) launch_chained(fold_kernel<true, false>, grid, 256, 0, st, s, d, n_out, tw, alpha, a2, ad, (size_t)0);
+        else launch_chained(fold_kernel<false, false>, grid, 256, 0, st, s, d, n_out, tw, alpha, a2, ad, (size_t)0);
     }
     STWO_LAUNCH_CHECK("fold_kernel");
     return STWO_OK;

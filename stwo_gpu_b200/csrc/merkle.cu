@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(256) merkle_layer_kernel(uint32_t log_size, co
                                                            const __grid_constant__ MerkleCols<CAP> cols,
                                                            const uint32_t *const *__restrict__ dev_cols,
                                                            uint32_t n_cols, uint4 *__restrict__ out, uint32_t one) {
+    chain_wait();
     // 32-bit node indices: at most 2^31 nodes, and i + the grid's stride stays below 2^32
     const uint32_t n = 1u << log_size;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -193,6 +194,7 @@ template <int THREADS>
 __global__ void __launch_bounds__(THREADS) merkle_tree_kernel(const __grid_constant__ TreeParams p, uint32_t one) {
     __shared__ uint4 thin[2][THREADS][2];
     __shared__ uint32_t next;
+    chain_wait();
     uint32_t b = 0, u = blockIdx.x;
     for (;;) {
         merkle_unit<THREADS>(p, p.band[b], u, thin, one);
@@ -268,7 +270,7 @@ int plan_tree_bands(uint32_t max_log, TreePlan &tp) {
 
 template <int THREADS>
 void launch_tree(const TreeParams &p, uint32_t blocks, uint32_t jobs, cudaStream_t st) {
-    merkle_tree_kernel<THREADS><<<dim3(blocks, jobs), THREADS, 0, st>>>(p, 1u);
+    launch_chained(merkle_tree_kernel<THREADS>, dim3(blocks, jobs), THREADS, 0, st, p, 1u);
 }
 
 template <int CAP>
@@ -278,11 +280,11 @@ void launch_layer(uint32_t log_size, const uint32_t *prev, const uint32_t *const
     if (!cols_on_device)
         for (uint32_t i = 0; i < n_cols; i++) mc.c[i] = cols[i];
     if (cols_on_device)
-        merkle_layer_kernel<true, CAP><<<blocks, 256, 0, st>>>(log_size, reinterpret_cast<const uint4 *>(prev), mc,
+        launch_chained(merkle_layer_kernel<true, CAP>, blocks, 256, 0, st, log_size, reinterpret_cast<const uint4 *>(prev), mc,
                                                                cols, n_cols, reinterpret_cast<uint4 *>(out), 1u);
     else
-        merkle_layer_kernel<false, CAP><<<blocks, 256, 0, st>>>(log_size, reinterpret_cast<const uint4 *>(prev), mc,
-                                                                nullptr, n_cols, reinterpret_cast<uint4 *>(out), 1u);
+        launch_chained(merkle_layer_kernel<false, CAP>, blocks, 256, 0, st, log_size, reinterpret_cast<const uint4 *>(prev), mc,
+                                                                (const uint32_t *const *)nullptr, n_cols, reinterpret_cast<uint4 *>(out), 1u);
 }
 
 }  // namespace

@@ -23,6 +23,7 @@ namespace {
 struct Acc4 { uint32_t *l[4]; const uint32_t *r[4]; };
 
 __global__ void accumulate_kernel(const __grid_constant__ Acc4 p, uint64_t n4, uint64_t n) {
+    chain_wait();
     for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < n4; k += (uint64_t)gridDim.x * blockDim.x) {
 #pragma unroll
         for (int c = 0; c < 4; c++) {
@@ -67,6 +68,7 @@ struct WideFibParams {
 // group of four columns: a folded sum plus at most four products stays below 2^64.
 template <int CAP>
 __global__ void __launch_bounds__(256, 4) wide_fib_kernel(const __grid_constant__ WideFibParams<CAP> p) {
+    chain_wait();
     const uint64_t n = 1ull << p.log_size;
     const uint64_t pairs = (n + 1) / 2;
     // The column pointers and each column's power, staged once per CTA: the column loop
@@ -196,6 +198,7 @@ __device__ __forceinline__ uint32_t qcoord(const qm31 &v, uint32_t q) {
 
 template <int CAP>
 __global__ void __launch_bounds__(WTC_THREADS, 3) wide_fib_tc_kernel(const __grid_constant__ WideFibParams<CAP> p) {
+    chain_wait();
     constexpr int N = 16;
     constexpr uint32_t SLOT = 32, TM_COLS = 64;
     constexpr uint32_t IDESC = tc::idesc_u8<128, N>();
@@ -433,7 +436,7 @@ bool launch_wf_tc(const WideFibParams<CAP> &p, uint32_t jobs, cudaStream_t st) {
         return false;
     const uint64_t tiles = 1ull << (p.log_size - 7), cap = 2ull * device_sm_count();
     const unsigned gx = (unsigned)(tiles < cap ? tiles : cap);
-    wide_fib_tc_kernel<CAP><<<dim3(gx, jobs), WTC_THREADS, wtc_smem_bytes(p.n_cols), st>>>(p);
+    launch_chained(wide_fib_tc_kernel<CAP>, dim3(gx, jobs), WTC_THREADS, wtc_smem_bytes(p.n_cols), st, p);
     return true;
 }
 
@@ -445,8 +448,8 @@ void launch_wf(const WideFibParams<CAP> &p, uint64_t pairs, uint32_t jobs, cudaS
     uint64_t blocks = (pairs + threads - 1) / threads, cap = (uint64_t)device_sm_count() * 32;
     if (blocks > cap) blocks = cap;
     // n_cols <= WF_MAX_COLS: at most 2048 x 24 bytes, the default dynamic limit.
-    wide_fib_kernel<CAP>
-        <<<dim3((unsigned)blocks, jobs), threads, (size_t)p.n_cols * (sizeof(qm31) + sizeof(void *)), st>>>(p);
+    launch_chained(wide_fib_kernel<CAP>, dim3((unsigned)blocks, jobs), threads,
+                   (size_t)p.n_cols * (sizeof(qm31) + sizeof(void *)), st, p);
 }
 
 template <int CAP>
@@ -516,7 +519,7 @@ int accumulate_async(uint32_t *const *left4, const uint32_t *const *right4, uint
     uint64_t n4 = (n + 3) / 4;
     uint64_t blocks = (n4 + 255) / 256, cap = (uint64_t)device_sm_count() * 16;
     if (blocks > cap) blocks = cap;
-    accumulate_kernel<<<(unsigned)blocks, 256, 0, st>>>(p, n4, n);
+    launch_chained(accumulate_kernel, (unsigned)blocks, 256, 0, st, p, n4, n);
     STWO_LAUNCH_CHECK("accumulate_kernel");
     return STWO_OK;
 }

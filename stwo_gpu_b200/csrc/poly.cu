@@ -29,6 +29,7 @@ struct TwiddleParams {
 };
 
 __global__ void twiddle_tree_kernel(const __grid_constant__ TwiddleParams p, uint32_t *tw) {
+    chain_wait();
     const uint64_t size = 1ull << p.m;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i + 1 < size;
          i += (uint64_t)gridDim.x * blockDim.x) {
@@ -67,7 +68,7 @@ int precompute_tree(cpoint initial, cpoint step, uint32_t m, uint32_t *tw, uint3
         dst = tmp;
     }
     uint32_t blocks = (uint32_t)std::min<uint64_t>((size + 255) / 256, (uint64_t)device_sm_count() * 16);
-    twiddle_tree_kernel<<<std::max(1u, blocks), 256, 0, st>>>(p, dst);
+    launch_chained(twiddle_tree_kernel, std::max(1u, blocks), 256, 0, st, p, dst);
     STWO_LAUNCH_CHECK("twiddle_tree_kernel");
     int rc = STWO_OK;
     if (itw) rc = batch_inverse_m31_async(dst, itw, size, st);
@@ -294,6 +295,7 @@ __device__ __forceinline__ void eap_body(uint32_t poly, uint32_t chunk, uint32_t
 // Three CTAs per SM: at four the per-polynomial factor tables read from the kernel
 // parameters spill (measured 3% slower over 32 x 2^22 coefficients).
 __global__ void __launch_bounds__(EAP_THREADS, 3) eval_at_point_kernel(const __grid_constant__ EapParams p) {
+    chain_wait();
     uint32_t poly = 0;
     while (poly + 1 < p.n_polys && blockIdx.x >= p.block_start[poly + 1]) poly++;
     const uint32_t chunk = blockIdx.x - p.block_start[poly];
@@ -315,6 +317,7 @@ __global__ void __launch_bounds__(EAP_THREADS, 4) eval_at_point_dev_kernel(const
                                                                            uint32_t n_polys, uint32_t iter_log,
                                                                            const qm31 *point, qm31 *partials,
                                                                            uint32_t *tickets, qm31 *results, size_t js) {
+    chain_wait();
     // blockIdx.y: the job, whose descriptors, point, partials, tickets and results are
     // job 0's moved by blockIdx.y * js bytes
     polys = job_ptr(polys, js, blockIdx.y);
@@ -429,7 +432,7 @@ int eval_at_points_async(const uint32_t *const *coeffs, const uint32_t *log_size
         p.partials = partials + part_off;
         p.tickets = tickets + done;
         p.results = reinterpret_cast<qm31 *>(results) + done;
-        eval_at_point_kernel<<<b, EAP_THREADS, 0, st>>>(p);
+        launch_chained(eval_at_point_kernel, b, EAP_THREADS, 0, st, p);
         STWO_LAUNCH_CHECK("eval_at_point_kernel");
         part_off += b;
         done += cnt;
@@ -449,7 +452,7 @@ int eval_at_points_dev_async(const void *polys_dev, uint32_t n_polys, uint32_t i
     STWO_REQUIRE(jobs >= 1 && jobs <= 65535, STWO_ERR_INVALID_ARGUMENT, "eval_at_point sets per launch: %u", jobs);
     STWO_REQUIRE(iter_log >= (uint32_t)EAP_ITER_LOG_MIN && iter_log <= (uint32_t)EAP_ITER_LOG_MAX,
                  STWO_ERR_INVALID_ARGUMENT, "eval_at_point groups per CTA 2^%u", iter_log);
-    eval_at_point_dev_kernel<<<dim3(total_blocks, jobs), EAP_THREADS, 0, st>>>(
+    launch_chained(eval_at_point_dev_kernel, dim3(total_blocks, jobs), EAP_THREADS, 0, st,
         static_cast<const EapDevPoly *>(polys_dev), n_polys, iter_log, static_cast<const qm31 *>(point_dev),
         static_cast<qm31 *>(partials), tickets, static_cast<qm31 *>(results), js);
     STWO_LAUNCH_CHECK("eval_at_point_dev_kernel");

@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(256) wide_fib_trace_kernel(const uint32_t *__r
                                                              const uint32_t *__restrict__ a1,
                                                              uint32_t *const *__restrict__ cols, uint32_t n_cols,
                                                              uint64_t rows, size_t js) {
+    chain_wait();
     a0 = job_ptr(a0, js, blockIdx.y);
     a1 = job_ptr(a1, js, blockIdx.y);
     cols = job_ptr(cols, js, blockIdx.y);
@@ -161,6 +162,7 @@ inline void vanishing_inverses(uint32_t L, uint32_t out[2]) {
 // Channel step after the trace tree: mix its root, draw the composition coefficient r,
 // and write powers[k] = r^k (k < n_powers; lane l computes k = l, l + 32, ...).
 __global__ void fs_trace_kernel(ProofState *s, const uint32_t *root, qm31 *powers, uint32_t n_powers, size_t js) {
+    chain_wait();
     s = job_ptr(s, js, blockIdx.x);  // one CTA a job
     root = job_ptr(root, js, blockIdx.x);
     powers = job_ptr(powers, js, blockIdx.x);
@@ -184,6 +186,7 @@ __global__ void fs_trace_kernel(ProofState *s, const uint32_t *root, qm31 *power
 // Channel step after the composition tree: mix its root, draw t and take the OODS
 // point (CirclePoint::get_random_point): x = (1 - t^2) / (1 + t^2), y = 2t / (1 + t^2).
 __global__ void fs_comp_kernel(ProofState *s, const uint32_t *root, size_t js) {
+    chain_wait();
     s = job_ptr(s, js, blockIdx.x);  // one thread a job
     root = job_ptr(root, js, blockIdx.x);
     for (int i = 0; i < 8; i++) s->roots[1][i] = root[i];
@@ -208,6 +211,7 @@ constexpr uint32_t OODS_STAGED = 1024;
 __global__ void __launch_bounds__(256) fs_oods_kernel(ProofState *s, const qm31 *sampled, const qm31 *powers,
                                                       uint32_t N, uint32_t L, cpoint vsh, QuotParamsDev *q_comp,
                                                       QuotParamsDev *q_trace, size_t js) {
+    chain_wait();
     s = job_ptr(s, js, blockIdx.x);  // one CTA a job
     sampled = job_ptr(sampled, js, blockIdx.x);
     powers = job_ptr(powers, js, blockIdx.x);
@@ -258,6 +262,7 @@ __global__ void __launch_bounds__(256) fs_oods_kernel(ProofState *s, const qm31 
 // Channel step after an FRI tree: mix its root, draw the folding alpha.
 __global__ void fs_layer_kernel(ProofState *s, const uint32_t *root, uint32_t root_slot, uint32_t alpha_slot,
                                 size_t js) {
+    chain_wait();
     s = job_ptr(s, js, blockIdx.x);  // one thread a job
     root = job_ptr(root, js, blockIdx.x);
     for (int i = 0; i < 8; i++) s->roots[root_slot][i] = root[i];
@@ -323,6 +328,7 @@ struct TailParams {
 
 __global__ void __launch_bounds__(TAIL_THREADS) fri_tail_kernel(ProofState *s, const TailParams *__restrict__ tp,
                                                                  uint32_t one, size_t js) {
+    chain_wait();
     s = job_ptr(s, js, blockIdx.x);  // one CTA a job; the job's parameters hold its own pointers
     tp = job_ptr(tp, js, blockIdx.x);
     extern __shared__ uint4 t_buf[];
@@ -429,7 +435,7 @@ int launch_fri_tail(ProofState *s, const TailParams *tp, uint32_t jobs, size_t j
         return (int)STWO_OK;
     });
     if (rc) return rc;
-    fri_tail_kernel<<<jobs, TAIL_THREADS, TAIL_SMEM, st>>>(s, tp, 1u, js);
+    launch_chained(fri_tail_kernel, jobs, TAIL_THREADS, TAIL_SMEM, st, s, tp, 1u, js);
     STWO_LAUNCH_CHECK("fri_tail_kernel");
     return STWO_OK;
 }
@@ -448,6 +454,7 @@ __device__ __forceinline__ uint32_t ctz128(const uint32_t w[4]) {
 }
 
 __global__ void __launch_bounds__(256) grind_kernel(ProofState *s, uint32_t pow_bits, uint64_t max_k, size_t js) {
+    chain_wait();
     s = job_ptr(s, js, blockIdx.y);
     const uint32_t one = 1;
     uint32_t d[8];
@@ -475,6 +482,7 @@ __global__ void __launch_bounds__(256) grind_kernel(ProofState *s, uint32_t pow_
 // After the search: mix the nonce and draw the raw query words (Queries::generate takes
 // each u32 masked to the largest domain's log size).
 __global__ void fs_finish_kernel(ProofState *s, uint32_t n_queries, size_t js) {
+    chain_wait();
     s = job_ptr(s, js, blockIdx.x);  // one thread a job
     if (s->nonce == ~0ull) {
         s->error |= fs::ERR_GRIND;
@@ -495,6 +503,7 @@ struct GatherReq {
 };
 
 __global__ void gather_kernel(const GatherReq *__restrict__ req, uint32_t n, uint32_t *__restrict__ out) {
+    chain_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = req[i].ptr[req[i].idx];
 }
@@ -635,7 +644,7 @@ struct Gatherer {
         memcpy(stage, reqs.data(), req_bytes);
         uint32_t *out_stage = reinterpret_cast<uint32_t *>(static_cast<uint8_t *>(stage) + req_bytes);
         STWO_CUDA_TRY(cudaMemcpyAsync(dreq, stage, req_bytes, cudaMemcpyHostToDevice, st));
-        gather_kernel<<<(unsigned)((reqs.size() + 255) / 256), 256, 0, st>>>(dreq, (uint32_t)reqs.size(), dout);
+        launch_chained(gather_kernel, (unsigned)((reqs.size() + 255) / 256), 256, 0, st, dreq, (uint32_t)reqs.size(), dout);
         STWO_LAUNCH_CHECK("gather_kernel");
         STWO_CUDA_TRY(cudaMemcpyAsync(out_stage, dout, reqs.size() * 4, cudaMemcpyDeviceToHost, st));
         PV_TRY(wait_stream(st));
@@ -1164,7 +1173,7 @@ int prove_jobs(const Job &j, uint32_t K, const uint32_t *const *a0_in, const uin
             const uint32_t threads = rows < (uint64_t)device_sm_count() * 256 ? 64 : 256;
             const uint64_t blocks =
                 std::min<uint64_t>((rows + threads - 1) / threads, (uint64_t)device_sm_count() * 16);
-            wide_fib_trace_kernel<<<dim3((unsigned)blocks, K), threads, 0, st>>>(
+            launch_chained(wide_fib_trace_kernel, dim3((unsigned)blocks, K), threads, 0, st,
                 a0, a1, reinterpret_cast<uint32_t *const *>(dev_at(off_tpoly)), N, rows, js);
             STWO_LAUNCH_CHECK("wide_fib_trace_kernel");
         }
@@ -1176,7 +1185,7 @@ int prove_jobs(const Job &j, uint32_t K, const uint32_t *const *a0_in, const uin
                                          t.n_tickets, K, js, st);
         };
         PV_TRY(commit(t_trace));
-        fs_trace_kernel<<<K, 32, 0, st>>>(dstate, t_trace.layers[0], powers, N - 2, js);
+        launch_chained(fs_trace_kernel, K, 32, 0, st, dstate, t_trace.layers[0], powers, N - 2, js);
         STWO_LAUNCH_CHECK("fs_trace_kernel");
         PV_TRY(record(1, capturing));
 
@@ -1189,14 +1198,14 @@ int prove_jobs(const Job &j, uint32_t K, const uint32_t *const *a0_in, const uin
         PV_TRY(fft_all(comp, comp, E, E, itw, true, nullptr));  // in place -> coefficients
         PV_TRY(fft_all(comp, cev, D, E, tw, false, nullptr));
         PV_TRY(commit(t_comp));
-        fs_comp_kernel<<<K, 1, 0, st>>>(dstate, t_comp.layers[0], js);
+        launch_chained(fs_comp_kernel, K, 1, 0, st, dstate, t_comp.layers[0], js);
         STWO_LAUNCH_CHECK("fs_comp_kernel");
         PV_TRY(record(2, capturing));
 
         // ---- 3. out-of-domain sampling
         PV_TRY(eval_at_points_dev_async(dev_at(off_eap), eap_n, eap_iter, eap_total, dstate->oods, dsampled,
                                         eap_partials, dtickets, K, js, st));
-        fs_oods_kernel<<<K, 256, 0, st>>>(dstate, dsampled, powers, N, L, vanishing_shift(L), dqc, dqt, js);
+        launch_chained(fs_oods_kernel, K, 256, 0, st, dstate, dsampled, powers, N, L, vanishing_shift(L), dqc, dqt, js);
         STWO_LAUNCH_CHECK("fs_oods_kernel");
         PV_TRY(record(3, capturing));
 
@@ -1204,7 +1213,7 @@ int prove_jobs(const Job &j, uint32_t K, const uint32_t *const *a0_in, const uin
         PV_TRY(quotients_dev_async(dqc, D, 4, K, js, st));
         PV_TRY(quotients_dev_async(dqt, L + B, N, K, js, st));
         PV_TRY(commit(t_fri0));
-        fs_layer_kernel<<<K, 1, 0, st>>>(dstate, t_fri0.layers[0], 2, 0, js);
+        launch_chained(fs_layer_kernel, K, 1, 0, st, dstate, t_fri0.layers[0], 2u, 0u, js);
         STWO_LAUNCH_CHECK("fs_layer_kernel");
         for (int k = 0; k < 4; k++) {
             if (K == 1) STWO_CUDA_TRY(cudaMemsetAsync(lay[0][k], 0, 4ull << (D - 1), st));
@@ -1224,7 +1233,7 @@ int prove_jobs(const Job &j, uint32_t K, const uint32_t *const *a0_in, const uin
                                   st, &dstate->alphas[li], K, js));
             }
             PV_TRY(commit(t_lay[li]));
-            fs_layer_kernel<<<K, 1, 0, st>>>(dstate, t_lay[li].layers[0], 3 + li, li + 1, js);
+            launch_chained(fs_layer_kernel, K, 1, 0, st, dstate, t_lay[li].layers[0], 3 + li, li + 1, js);
             STWO_LAUNCH_CHECK("fs_layer_kernel");
             std::vector<const uint32_t *> s(lay[li].begin(), lay[li].end());
             PV_TRY(fold_async(s.data(), 1ull << lg, stwo_qm31{}, itw, tsz - (1ull << lg), lay[li + 1].data(), false, st,
@@ -1240,9 +1249,9 @@ int prove_jobs(const Job &j, uint32_t K, const uint32_t *const *a0_in, const uin
                 std::max<uint64_t>(256, std::min<uint64_t>(want, (uint64_t)device_sm_count() * 1024));
             const uint64_t blocks = (threads + 255) / 256, grid = blocks * 256;
             const uint64_t max_k = ((1ull << (j.pow_bits + 6)) + grid - 1) / grid + 1;  // gives up after 2^(pow_bits+6)
-            grind_kernel<<<dim3((unsigned)blocks, K), 256, 0, st>>>(dstate, j.pow_bits, max_k, js);
+            launch_chained(grind_kernel, dim3((unsigned)blocks, K), 256, 0, st, dstate, j.pow_bits, max_k, js);
             STWO_LAUNCH_CHECK("grind_kernel");
-            fs_finish_kernel<<<K, 1, 0, st>>>(dstate, j.n_queries, js);
+            launch_chained(fs_finish_kernel, K, 1, 0, st, dstate, j.n_queries, js);
             STWO_LAUNCH_CHECK("fs_finish_kernel");
         }
         return STWO_OK;

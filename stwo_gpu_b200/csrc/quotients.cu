@@ -99,6 +99,7 @@ template <bool COLS_ON_DEVICE, int NB, class PR>
 __global__ void __launch_bounds__(256, QUOT_MIN_BLOCKS) quotients_kernel(const __grid_constant__ PR pr,
                                                                          const uint32_t *const *__restrict__ dev_cols,
                                                                          uint32_t n_stage, uint32_t two) {
+    chain_wait();
     const auto &p = pr.get();
     extern __shared__ uint4 q_smem[];
     qm31 *s_c2 = reinterpret_cast<qm31 *>(q_smem);
@@ -265,6 +266,7 @@ __host__ __device__ constexpr size_t qtc_smem_bytes(uint32_t c8, int nb) {
 template <int NB, bool COLS_ON_DEVICE, class PR>
 __global__ void __launch_bounds__(QTC_THREADS, 2)
     quotients_tc_kernel(const __grid_constant__ PR pr, const uint32_t *const *__restrict__ dev_cols, uint32_t n_cols) {
+    chain_wait();
     constexpr int N = 16 * NB;
     // two accumulators, each an even-row half and an odd-row half of N columns, every
     // half at a multiple of 32 columns
@@ -549,7 +551,7 @@ int launch_quot_tc(const PR &pr, const uint32_t *const *dev_cols, uint32_t n_col
     // shared memory keep such CTAs to two an SM, so the SM's 512 columns always suffice.
     size_t smem = qtc_smem_bytes(c8, NB);
     if (NB >= 3 && smem < QTC_SMEM_FLOOR) smem = QTC_SMEM_FLOOR;
-    kern<<<dim3(gx, jobs), QTC_THREADS, smem, st>>>(pr, dev_cols, n_cols);
+    launch_chained(kern, dim3(gx, jobs), QTC_THREADS, smem, st, pr, dev_cols, n_cols);
     STWO_LAUNCH_CHECK("quotients_tc_kernel");
     return STWO_OK;
 }
@@ -659,10 +661,12 @@ int quotients_async(uint32_t half_init, uint32_t half_step, uint32_t log_size, c
     const size_t smem = (size_t)n_stage * (sizeof(qm31) + sizeof(void *));
     auto launch = [&](auto nb) {
         constexpr int NBV = decltype(nb)::value;
+        using PR = std::decay_t<decltype(*holder)>;
         if (cols_on_device)
-            quotients_kernel<true, NBV><<<(unsigned)blocks, 256, smem, st>>>(*holder, cols, n_stage, 2u);
+            launch_chained(quotients_kernel<true, NBV, PR>, (unsigned)blocks, 256, smem, st, *holder, cols, n_stage, 2u);
         else
-            quotients_kernel<false, NBV><<<(unsigned)blocks, 256, smem, st>>>(*holder, nullptr, n_stage, 2u);
+            launch_chained(quotients_kernel<false, NBV, PR>, (unsigned)blocks, 256, smem, st, *holder,
+                           (const uint32_t *const *)nullptr, n_stage, 2u);
     };
     switch (n_batches) {
     case 1: launch(std::integral_constant<int, 1>{}); break;
@@ -689,8 +693,8 @@ int quotients_dev_async(const QuotParamsDev *p_dev, uint32_t log_size, uint32_t 
     uint64_t blocks = (pairs + 255) / 256;
     uint64_t cap = (uint64_t)device_sm_count() * 8;
     if (blocks > cap) blocks = cap;
-    quotients_kernel<false, 1><<<dim3((unsigned)blocks, jobs), 256, smem, st>>>(QuotByRef{p_dev, js}, nullptr, n_stage,
-                                                                               2u);
+    launch_chained(quotients_kernel<false, 1, QuotByRef>, dim3((unsigned)blocks, jobs), 256, smem, st,
+                   QuotByRef{p_dev, js}, (const uint32_t *const *)nullptr, n_stage, 2u);
     STWO_LAUNCH_CHECK("quotients_kernel");
     return STWO_OK;
 }
