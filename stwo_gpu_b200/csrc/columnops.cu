@@ -8,13 +8,9 @@
 // the other, so every HBM access is a full line and in-place is safe.
 //
 // Batch inverse (reference: per-block product tree in shared memory,
-// cuda/src/batch_inverse.cu:25-155). Here each warp owns 256 elements with
-// coalesced accesses (lane l takes elements l, l+32, ...): prefix products in
-// registers, a multiplicative scan of the lane products in both directions with
-// shuffles, one field inversion of the warp product (computed by every lane, so no
-// barrier is needed) and back-substitution: 3 multiplications per element and one
-// inversion per 256 elements. QM31 elements are inverted through their M31 norms, so
-// the scan and its products stay in M31.
+// cuda/src/batch_inverse.cu:25-155). Here each thread inverts the product of its own 8 or
+// 16 elements (a warp's accesses are whole lines) and unwinds it: no shared memory, no
+// barrier, no shuffles. QM31 elements are inverted through their M31 norms.
 #include <map>
 #include <mutex>
 #include <vector>
@@ -71,121 +67,89 @@ __global__ void __launch_bounds__(256) bitrev_tiled_kernel(uint32_t *a, uint32_t
 }
 
 // ---------------------------------------------------------------- batch inverse
-constexpr int BI_THREADS = 256;
-constexpr int BI_PER_THREAD = 8;
+constexpr int BI_THREADS = 128;
+constexpr int BI_M31_PER_THREAD = 16;
+constexpr int BI_QM31_PER_THREAD = 8;
 
-template <typename F>
-struct FieldT;
-template <>
-struct FieldT<uint32_t> {
-    __device__ static uint32_t one() { return 1u; }
-    __device__ static uint32_t mul(uint32_t a, uint32_t b) { return m31_mul(a, b); }
-    __device__ static uint32_t inv(uint32_t a) { return m31_inv(a); }
-    __device__ static uint32_t shfl_up(uint32_t v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
-    __device__ static uint32_t shfl_down(uint32_t v, int d) { return __shfl_down_sync(0xffffffffu, v, d); }
-};
-
-// Warp-level Montgomery batch inverse: each warp owns 32 x BI_PER_THREAD elements,
-// lane l holding elements base + i*32 + l (coalesced loads and stores). Prefix
-// products in registers, inclusive scans of the lane products in both directions
-// with shuffles, and one field inversion of the warp product per warp (computed
-// redundantly by every lane, so there is no barrier and no shared memory).
-template <typename F>
-__global__ void __launch_bounds__(BI_THREADS) batch_inverse_kernel(const F *__restrict__ src, F *__restrict__ dst,
-                                                                    uint64_t n) {
+// Montgomery's batch inverse with a thread's own elements as the batch: prefix products in
+// registers, one field inversion of the thread's product (30 squarings and 8 products,
+// 2.4 an element), and the inverses unwound from the last element down. A warp's elements
+// are base + i * 32 + lane, so loads and stores are whole lines; no lane needs another's
+// values. (A warp-wide product with one inversion, computed by every lane all the same,
+// cost the same instructions plus two shuffle scans on the critical path: 4 x 9999991
+// values 100 us, against 82 us with 8 elements a thread and 72 us with 16.)
+__global__ void __launch_bounds__(BI_THREADS) batch_inverse_m31_kernel(const uint32_t *__restrict__ src,
+                                                                       uint32_t *__restrict__ dst, uint64_t n) {
     chain_wait();
-    using T = FieldT<F>;
+    constexpr int E = BI_M31_PER_THREAD;
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t warp_global = ((uint64_t)blockIdx.x * BI_THREADS + threadIdx.x) >> 5;
-    const uint64_t base = warp_global * (32 * BI_PER_THREAD) + lane;
-    F v[BI_PER_THREAD], pre[BI_PER_THREAD];
-    F run = T::one();
+    const uint64_t base = warp_global * (32 * E) + lane;
+    uint32_t v[E], pre[E];
+    uint32_t run = 1;
 #pragma unroll
-    for (int i = 0; i < BI_PER_THREAD; i++) {
+    for (int i = 0; i < E; i++) {
         const uint64_t idx = base + (uint64_t)i * 32;
-        v[i] = (idx < n) ? src[idx] : T::one();
-        run = T::mul(run, v[i]);
+        v[i] = (idx < n) ? src[idx] : 1u;
+        run = m31_mul(run, v[i]);
         pre[i] = run;
     }
-    // Inclusive scans of lane products, forward (prefix) and backward (suffix).
-    F inc = run, suf = run;
+    uint32_t r = m31_inv(run);
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        F u = T::shfl_up(inc, d);
-        F w = T::shfl_down(suf, d);
-        if (lane >= (uint32_t)d) inc = T::mul(inc, u);
-        if (lane + d < 32u) suf = T::mul(suf, w);
-    }
-    const F total = T::shfl_down(inc, 31 - lane);  // lane 31's inclusive prefix, broadcast via shuffles
-    F ex_pre = T::shfl_up(inc, 1), ex_suf = T::shfl_down(suf, 1);
-    if (lane == 0) ex_pre = T::one();
-    if (lane == 31) ex_suf = T::one();
-    // inverse of this lane's product = inv(total) * (product before) * (product after)
-    F r = T::mul(T::inv(total), T::mul(ex_pre, ex_suf));
-#pragma unroll
-    for (int i = BI_PER_THREAD - 1; i >= 0; i--) {
-        F inv_i = i > 0 ? T::mul(r, pre[i - 1]) : r;
+    for (int i = E - 1; i >= 0; i--) {
+        const uint32_t inv_i = i > 0 ? m31_mul(r, pre[i - 1]) : r;
         const uint64_t idx = base + (uint64_t)i * 32;
         if (idx < n) dst[idx] = inv_i;
-        r = T::mul(r, v[i]);
+        r = m31_mul(r, v[i]);
     }
 }
 
 // QM31 batch inverse through norms. For z = a + b u (a, b in CM31, u^2 = R = 2 + i):
 // z (a - b u) = a^2 - R b^2 = N in CM31, and N conj(N) = |N|^2 in M31, so
-// z^-1 = (a - b u) conj(N) / |N|^2. The warp's Montgomery inverse then runs on the
-// M31 norms (three M31 products an element, one-word shuffles, one M31 inversion a
-// warp) instead of on QM31 values (three QM31 products an element); the inverse is
-// unique, so the values are the same.
-__global__ void __launch_bounds__(BI_THREADS) batch_inverse_qm31_norm_kernel(const qm31 *__restrict__ src,
-                                                                             qm31 *__restrict__ dst, uint64_t n) {
+// z^-1 = (a - b u) conj(N) / |N|^2. A thread's Montgomery inverse then runs on the
+// M31 norms of its elements instead of on QM31 values; the inverse is unique, so the
+// values are the same. Bound by instruction issue next to HBM (32 bytes an element): no
+// shuffle scans (as above), CM31 products as two-term dot products with one three-
+// instruction reduction (m31_dot2), and 72 registers for seven CTAs of 128 threads an SM.
+// 9999991 elements: 86.1 -> 65.5 us, 2^24: 139 -> 103 us (5.2 TB/s, 80% of the measured
+// copy rate); 6 elements a thread 65.6, 4: 71.6, 12: 68.5; CTAs of 256 threads 67.6-69.6.
+__global__ void __launch_bounds__(BI_THREADS, 7) batch_inverse_qm31_norm_kernel(const qm31 *__restrict__ src,
+                                                                                qm31 *__restrict__ dst, uint64_t n) {
     chain_wait();
+    constexpr int E = BI_QM31_PER_THREAD;
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t warp_global = ((uint64_t)blockIdx.x * BI_THREADS + threadIdx.x) >> 5;
-    const uint64_t base = warp_global * (32 * BI_PER_THREAD) + lane;
-    qm31 v[BI_PER_THREAD];
-    cm31 nrm[BI_PER_THREAD];
-    uint32_t pre[BI_PER_THREAD], mag[BI_PER_THREAD];
+    const uint64_t base = warp_global * (32 * E) + lane;
+    qm31 v[E];
+    cm31 nrm[E];
+    uint32_t pre[E], mag[E];
     uint32_t run = 1;
 #pragma unroll
-    for (int i = 0; i < BI_PER_THREAD; i++) {
+    for (int i = 0; i < E; i++) {
         const uint64_t idx = base + (uint64_t)i * 32;
         v[i] = (idx < n) ? src[idx] : qm31_one();
         const cm31 a2 = cm31_sqr(v[i].a), b2 = cm31_sqr(v[i].b);
         const cm31 rb2 = {m31_sub(m31_add(b2.a, b2.a), b2.b), m31_add(m31_add(b2.b, b2.b), b2.a)};  // R b^2
         nrm[i] = cm31_sub(a2, rb2);
-        mag[i] = reduce64_p((uint64_t)nrm[i].a * nrm[i].a + (uint64_t)nrm[i].b * nrm[i].b);
+        mag[i] = m31_dot2(nrm[i].a, nrm[i].a << 1, nrm[i].b, nrm[i].b << 1);
         run = m31_mul(run, mag[i]);
         pre[i] = run;
     }
-    // Inclusive scans of the lanes' norm products, forward (prefix) and backward (suffix).
-    uint32_t inc = run, suf = run;
+    uint32_t r = m31_inv(run);
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t u = __shfl_up_sync(0xffffffffu, inc, d);
-        const uint32_t w = __shfl_down_sync(0xffffffffu, suf, d);
-        if (lane >= (uint32_t)d) inc = m31_mul(inc, u);
-        if (lane + d < 32u) suf = m31_mul(suf, w);
-    }
-    const uint32_t total = __shfl_down_sync(0xffffffffu, inc, 31 - lane);
-    uint32_t ex_pre = __shfl_up_sync(0xffffffffu, inc, 1), ex_suf = __shfl_down_sync(0xffffffffu, suf, 1);
-    if (lane == 0) ex_pre = 1;
-    if (lane == 31) ex_suf = 1;
-    uint32_t r = m31_mul(m31_inv(total), m31_mul(ex_pre, ex_suf));
-#pragma unroll
-    for (int i = BI_PER_THREAD - 1; i >= 0; i--) {
+    for (int i = E - 1; i >= 0; i--) {
         const uint32_t minv = i > 0 ? m31_mul(r, pre[i - 1]) : r;  // 1 / |N_i|^2
         const uint64_t idx = base + (uint64_t)i * 32;
         r = m31_mul(r, mag[i]);
         // 1 / N_i = c + d i with c = N.a / |N|^2, d = -N.b / |N|^2; the products
-        // (x + y i)(c + d i) = (x c + y (p - d)) + (x d + y c) i reduced once each
-        const uint32_t c = m31_mul(nrm[i].a, minv), nd = m31_mul(nrm[i].b, minv), d = m31_neg(nd);
+        // (x + y i)(c + d i) = (x c + y (p - d)) + (x d + y c) i reduced once each, and
+        // negated for the u part by the coefficients (p - c, p - d)
+        const uint32_t c = m31_mul(nrm[i].a, minv), nd = m31_mul(nrm[i].b, minv);
+        const uint32_t c2 = c << 1, nd2 = nd << 1, d2 = (P - nd) << 1, nc2 = (P - c) << 1;
         const qm31 z = v[i];
-        const cm31 lo = {reduce64_p((uint64_t)z.a.a * c + (uint64_t)z.a.b * nd),
-                         reduce64_p((uint64_t)z.a.a * d + (uint64_t)z.a.b * c)};
-        const cm31 hi = {reduce64_p((uint64_t)z.b.a * c + (uint64_t)z.b.b * nd),
-                         reduce64_p((uint64_t)z.b.a * d + (uint64_t)z.b.b * c)};
-        if (idx < n) dst[idx] = {lo, cm31_neg(hi)};
+        const cm31 lo = {m31_dot2(z.a.a, c2, z.a.b, nd2), m31_dot2(z.a.a, d2, z.a.b, c2)};
+        const cm31 nhi = {m31_dot2(z.b.a, nc2, z.b.b, d2), m31_dot2(z.b.a, nd2, z.b.b, nc2)};
+        if (idx < n) dst[idx] = {lo, nhi};
     }
 }
 
@@ -236,15 +200,15 @@ int bit_reverse_async(uint32_t *col, uint64_t n, uint32_t words, cudaStream_t st
 
 int batch_inverse_m31_async(const uint32_t *src, uint32_t *dst, uint64_t n, cudaStream_t st) {
     if (n == 0) return STWO_OK;
-    uint64_t blocks = (n + BI_THREADS * BI_PER_THREAD - 1) / (BI_THREADS * BI_PER_THREAD);
-    launch_chained(batch_inverse_kernel<uint32_t>, (unsigned)blocks, BI_THREADS, 0, st, src, dst, n);
-    STWO_LAUNCH_CHECK("batch_inverse_kernel<m31>");
+    uint64_t blocks = (n + BI_THREADS * BI_M31_PER_THREAD - 1) / (BI_THREADS * BI_M31_PER_THREAD);
+    launch_chained(batch_inverse_m31_kernel, (unsigned)blocks, BI_THREADS, 0, st, src, dst, n);
+    STWO_LAUNCH_CHECK("batch_inverse_m31_kernel");
     return STWO_OK;
 }
 
 int batch_inverse_qm31_async(const uint32_t *src, uint32_t *dst, uint64_t n, cudaStream_t st) {
     if (n == 0) return STWO_OK;
-    uint64_t blocks = (n + BI_THREADS * BI_PER_THREAD - 1) / (BI_THREADS * BI_PER_THREAD);
+    uint64_t blocks = (n + BI_THREADS * BI_QM31_PER_THREAD - 1) / (BI_THREADS * BI_QM31_PER_THREAD);
     launch_chained(batch_inverse_qm31_norm_kernel, (unsigned)blocks, BI_THREADS, 0, st, reinterpret_cast<const qm31 *>(src),
                                                                             reinterpret_cast<qm31 *>(dst), n);
     STWO_LAUNCH_CHECK("batch_inverse_qm31_norm_kernel");

@@ -86,6 +86,14 @@ __host__ __device__ __forceinline__ uint32_t reduce64_p(uint64_t acc) {
     return reduce_once((uint32_t)s);
 }
 
+// x c + y d, canonical, for canonical x, y and doubled coefficients c2 = 2 c, d2 = 2 d with
+// c, d <= P: the sum 2 (x c + y d) stays below 2^64, its high word reduced once is below
+// P, and the halved low word adds at most P, as in m31_mul2.
+__host__ __device__ __forceinline__ uint32_t m31_dot2(uint32_t x, uint32_t c2, uint32_t y, uint32_t d2) {
+    const uint64_t w = (uint64_t)x * c2 + (uint64_t)y * d2;
+    return reduce_once(reduce_once((uint32_t)(w >> 32)) + ((uint32_t)w >> 1));
+}
+
 __host__ __device__ __forceinline__ uint32_t m31_sqr(uint32_t a) { return m31_mul(a, a); }
 
 __host__ __device__ inline uint32_t m31_pow(uint32_t a, uint64_t e) {
