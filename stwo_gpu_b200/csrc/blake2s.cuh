@@ -57,36 +57,74 @@ __device__ __forceinline__ uint32_t add2(uint32_t c, uint32_t d, uint32_t one) {
     return c + d;
 }
 
-#define STWO_G(a, b, c, d, x, y)    \
-    a = add3<FMA>(a, (x), b, one);  \
-    d = rotr16(d ^ a);              \
-    c = add2<FMA>(c, d, one);       \
-    b = rotr(b ^ c, 12);            \
-    a = add3<FMA>(a, (y), b, one);  \
-    d = rotr8(d ^ a);               \
-    c = add2<FMA>(c, d, one);       \
+// a + m[S] + b for a message whose words from W on are zero: no addition for those.
+template <bool FMA, int W, int S>
+__device__ __forceinline__ uint32_t add_msg(uint32_t a, const uint32_t *m, uint32_t b, uint32_t one) {
+    if constexpr (S < W) return add3<FMA>(a, m[S], b, one);
+    else return add2<FMA>(a, b, one);
+}
+
+#define STWO_G(a, b, c, d, s, t)          \
+    a = add_msg<FMA, W, s>(a, m, b, one); \
+    d = rotr16(d ^ a);                    \
+    c = add2<FMA>(c, d, one);             \
+    b = rotr(b ^ c, 12);                  \
+    a = add_msg<FMA, W, t>(a, m, b, one); \
+    d = rotr8(d ^ a);                     \
+    c = add2<FMA>(c, d, one);             \
+    b = rotr(b ^ c, 7);
+
+// G of the first column step from a zero chaining state (a = b = 0): two additions and two
+// xors fewer.
+#define STWO_G0(a, b, c, d, s, t)         \
+    a = m[s];                             \
+    d = rotr16(d ^ a);                    \
+    c = add2<FMA>(c, d, one);             \
+    b = rotr(c, 12);                      \
+    a = add_msg<FMA, W, t>(a, m, b, one); \
+    d = rotr8(d ^ a);                     \
+    c = add2<FMA>(c, d, one);             \
     b = rotr(b ^ c, 7);
 
 // One BLAKE2s round with message permutation s0..s15 (RFC 7693 SIGMA rows).
 #define STWO_ROUND(s0, s1, s2, s3, s4, s5, s6, s7, s8, s9, s10, s11, s12, s13, s14, s15) \
-    { STWO_G(v0, v4, v8, v12, m[s0], m[s1])                                            \
-      STWO_G(v1, v5, v9, v13, m[s2], m[s3])                                            \
-      STWO_G(v2, v6, v10, v14, m[s4], m[s5])                                           \
-      STWO_G(v3, v7, v11, v15, m[s6], m[s7])                                           \
-      STWO_G(v0, v5, v10, v15, m[s8], m[s9])                                           \
-      STWO_G(v1, v6, v11, v12, m[s10], m[s11])                                         \
-      STWO_G(v2, v7, v8, v13, m[s12], m[s13])                                          \
-      STWO_G(v3, v4, v9, v14, m[s14], m[s15]) }
+    { STWO_G(v0, v4, v8, v12, s0, s1)                                            \
+      STWO_G(v1, v5, v9, v13, s2, s3)                                            \
+      STWO_G(v2, v6, v10, v14, s4, s5)                                           \
+      STWO_G(v3, v7, v11, v15, s6, s7)                                           \
+      STWO_G(v0, v5, v10, v15, s8, s9)                                           \
+      STWO_G(v1, v6, v11, v12, s10, s11)                                         \
+      STWO_G(v2, v7, v8, v13, s12, s13)                                          \
+      STWO_G(v3, v4, v9, v14, s14, s15) }
 
 // Compression with byte counter t (low word) and finalisation flag f0; the Merkle
 // hasher and the nonce mixing use t = f0 = 0.
-template <bool FMA = true>
-__device__ __forceinline__ void compress_tf(uint32_t h[8], const uint32_t m[16], uint32_t t, uint32_t f0,
-                                            uint32_t one) {
-    uint32_t v0 = h[0], v1 = h[1], v2 = h[2], v3 = h[3], v4 = h[4], v5 = h[5], v6 = h[6], v7 = h[7];
+// W: the message's words from W on are zero (and m has W words). H0: the chaining state is
+// zero (h is only written). X: the two halves of the working state are joined before h is
+// read; the same values, scheduled differently (the tree kernel's 256 x 2^16 trees 89.4 us
+// with it and 91.4 without, the one-layer kernel 686 and 679 us for 64 x 2^22).
+template <bool FMA = true, int W = 16, bool H0 = false, bool X = H0>
+__device__ __forceinline__ void compress_tf(uint32_t h[8], const uint32_t *m, uint32_t t, uint32_t f0, uint32_t one) {
+    uint32_t v0 = H0 ? 0u : h[0], v1 = H0 ? 0u : h[1], v2 = H0 ? 0u : h[2], v3 = H0 ? 0u : h[3];
+    uint32_t v4 = H0 ? 0u : h[4], v5 = H0 ? 0u : h[5], v6 = H0 ? 0u : h[6], v7 = H0 ? 0u : h[7];
     uint32_t v8 = IV[0], v9 = IV[1], v10 = IV[2], v11 = IV[3], v12 = IV[4] ^ t, v13 = IV[5], v14 = IV[6] ^ f0,
              v15 = IV[7];
-    STWO_ROUND(0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15)
+    static_assert(!H0 || W >= 8, "the first column step reads eight words");
+    if constexpr (H0) {
+        STWO_G0(v0, v4, v8, v12, 0, 1)
+        STWO_G0(v1, v5, v9, v13, 2, 3)
+        STWO_G0(v2, v6, v10, v14, 4, 5)
+        STWO_G0(v3, v7, v11, v15, 6, 7)
+    } else {
+        STWO_G(v0, v4, v8, v12, 0, 1)
+        STWO_G(v1, v5, v9, v13, 2, 3)
+        STWO_G(v2, v6, v10, v14, 4, 5)
+        STWO_G(v3, v7, v11, v15, 6, 7)
+    }
+    STWO_G(v0, v5, v10, v15, 8, 9)
+    STWO_G(v1, v6, v11, v12, 10, 11)
+    STWO_G(v2, v7, v8, v13, 12, 13)
+    STWO_G(v3, v4, v9, v14, 14, 15)
     STWO_ROUND(14, 10, 4, 8, 9, 15, 13, 6, 1, 12, 0, 2, 11, 7, 5, 3)
     STWO_ROUND(11, 8, 12, 0, 5, 2, 15, 13, 10, 14, 3, 6, 7, 1, 9, 4)
     STWO_ROUND(7, 9, 3, 1, 13, 12, 11, 14, 2, 6, 5, 10, 4, 0, 15, 8)
@@ -96,6 +134,12 @@ __device__ __forceinline__ void compress_tf(uint32_t h[8], const uint32_t m[16],
     STWO_ROUND(13, 11, 7, 14, 12, 1, 3, 9, 5, 0, 15, 4, 8, 6, 2, 10)
     STWO_ROUND(6, 15, 14, 9, 11, 3, 0, 8, 12, 2, 13, 7, 1, 4, 10, 5)
     STWO_ROUND(10, 2, 8, 4, 7, 6, 1, 5, 15, 11, 9, 14, 3, 12, 13, 0)
+    if (X) {
+        const uint32_t x[8] = {v0 ^ v8, v1 ^ v9, v2 ^ v10, v3 ^ v11, v4 ^ v12, v5 ^ v13, v6 ^ v14, v7 ^ v15};
+#pragma unroll
+        for (int i = 0; i < 8; i++) h[i] = H0 ? x[i] : h[i] ^ x[i];
+        return;
+    }
     h[0] ^= v0 ^ v8;
     h[1] ^= v1 ^ v9;
     h[2] ^= v2 ^ v10;
@@ -106,9 +150,9 @@ __device__ __forceinline__ void compress_tf(uint32_t h[8], const uint32_t m[16],
     h[7] ^= v7 ^ v15;
 }
 
-template <bool FMA = true>
-__device__ __forceinline__ void compress(uint32_t h[8], const uint32_t m[16], uint32_t one) {
-    compress_tf<FMA>(h, m, 0u, 0u, one);
+template <bool FMA = true, int W = 16, bool H0 = false, bool X = H0>
+__device__ __forceinline__ void compress(uint32_t h[8], const uint32_t *m, uint32_t one) {
+    compress_tf<FMA, W, H0, X>(h, m, 0u, 0u, one);
 }
 
 }  // namespace blake

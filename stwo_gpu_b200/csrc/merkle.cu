@@ -98,6 +98,16 @@ __global__ void __launch_bounds__(256) merkle_layer_kernel(uint32_t log_size, co
 //
 // With spread s a thread hashes 2^s bottom-level nodes, so a unit stays dense for s + 1
 // levels before its upper levels thin out.
+//
+// The compression is about 18 KB of straight-line code, and the kernel issues at its
+// ceiling (81% of the slots) where it is dense, so both the instructions and the number of
+// copies count. Layers of four columns (the QM31 columns of the composition and of FRI,
+// half of their trees' compressions) take a form without the 120 additions of zero words;
+// full and padded chunks share one copy. B200, us: 4 columns at each of 2^12..2^22 643 ->
+// 573, 4 x 2^22 427 -> 388, 4 x 2^20 145 -> 134, 101 x 2^18 (a padded chunk) 152 -> 137;
+// 64 x 2^22 897 -> 896. Further copies cost more than they save: a zero-state form for
+// leaves beside this one 412 at 4 x 2^22, an eight-word form 659 over the mixed tree; one
+// copy for children and chunks alike 929 at 64 x 2^22.
 constexpr int MERKLE_MAX_BANDS = 6;
 
 struct TreeBand {
@@ -162,21 +172,29 @@ __device__ __forceinline__ void merkle_unit(const TreeParams &p, const TreeBand 
                 for (int q = 0; q < 4; q++) {
                     m[4 * q] = v[q].x; m[4 * q + 1] = v[q].y; m[4 * q + 2] = v[q].z; m[4 * q + 3] = v[q].w;
                 }
-                compress(h, m, one);
+                compress<true, 16, true>(h, m, one);
             }
-            uint32_t c0 = 0;
-            for (; c0 + 16 <= nc; c0 += 16) {  // full chunks: no per-word bound checks
+            if (nc == 4) {  // a QM31 column: the message's last twelve words are zero
+                uint32_t m4[4];
 #pragma unroll
-                for (int w = 0; w < 16; w++) m[w] = __ldg(ct[c0 + w] + i);
-                compress(h, m, one);
-            }
-            if (c0 < nc) {  // the zero-padded last chunk
+                for (int w = 0; w < 4; w++) m4[w] = __ldg(ct[w] + i);
+                compress<true, 4, false, true>(h, m4, one);
+            } else {
+                // one loop for full chunks and the zero-padded last one (see above)
+#pragma unroll 1
+                for (uint32_t c0 = 0; c0 < nc; c0 += 16) {
+                    if (c0 + 16 <= nc) {  // no per-word bound checks
 #pragma unroll
-                for (int w = 0; w < 16; w++) {
-                    const uint32_t cw = c0 + w;
-                    m[w] = cw < nc ? __ldg(ct[cw] + i) : 0u;
+                        for (int w = 0; w < 16; w++) m[w] = __ldg(ct[c0 + w] + i);
+                    } else {
+#pragma unroll
+                        for (int w = 0; w < 16; w++) {
+                            const uint32_t cw = c0 + w;
+                            m[w] = cw < nc ? __ldg(ct[cw] + i) : 0u;
+                        }
+                    }
+                    compress<true, 16, false, true>(h, m, one);
                 }
-                compress(h, m, one);
             }
             const uint4 lo = make_uint4(h[0], h[1], h[2], h[3]), hi = make_uint4(h[4], h[5], h[6], h[7]);
             out[2 * i] = lo;

@@ -1,0 +1,25 @@
+"""The tree kernel at every kind of column count: four columns take their own compression
+(twelve zero message words), other counts full and zero-padded chunks in one loop. Each
+count at the leaves and, with children, at a dense and a thin inner layer; every layer
+equals the oracle's."""
+import pytest
+
+from helpers import m31, rng
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nc", [1, 3, 4, 5, 8, 15, 16, 17, 20, 32, 36])
+def test_tree_layers_match_oracle(stwo, oracle, nc):
+    L = stwo._lib
+    r = rng(3100 + nc)
+    logs = [11] * nc + [10] * nc + [3] * nc + [0] * nc
+    cols = [m31(r, 1 << lg) for lg in logs]
+    bufs = [stwo.BaseFieldVec.from_numpy(c) for c in cols]
+    layers = [stwo.BaseFieldVec.new_uninitialized(8 << l) for l in range(12)]
+    L.check(L.lib().stwo_merkle_commit_tree(L.ptr_array([b.device_ptr for b in bufs]), L.u32_array(logs), len(logs),
+                                            11, L.ptr_array([x.device_ptr for x in layers]), None))
+    L.check(L.lib().stwo_stream_synchronize(None))
+    want = oracle.merkle_commit(cols)
+    for l in range(12):
+        assert (layers[l].to_numpy().reshape(-1, 8) == want[l]).all(), l
