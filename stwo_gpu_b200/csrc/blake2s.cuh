@@ -42,48 +42,48 @@ __device__ __forceinline__ uint32_t add_on_fma(uint32_t c, uint32_t d, uint32_t 
     return r;
 }
 
-// FMA: the additions as multiply-adds on the FMA pipe, for many threads hashing at
-// once (the xors and rotations keep the ALU pipe busy). Otherwise the three-input
-// a + b + m and c + d on the ALU pipe: two instructions fewer a G, for one thread
-// hashing alone (the device channel), whose time is its own instruction stream.
-template <bool FMA>
-__device__ __forceinline__ uint32_t add3(uint32_t a, uint32_t x, uint32_t b, uint32_t one) {
-    if (FMA) return add_on_fma(add_on_fma(a, x, one), b, one);
-    return a + x + b;
-}
-template <bool FMA>
-__device__ __forceinline__ uint32_t add2(uint32_t c, uint32_t d, uint32_t one) {
-    if (FMA) return add_on_fma(c, d, one);
-    return c + d;
-}
+// Where the additions of G go:
+//  * ADD_FMA: all on the FMA pipe, for many threads hashing at once (the xors and rotations
+//    keep the ALU pipe busy);
+//  * ADD_MIXED: half of them, for one thread or warp hashing alone (the device channel, the
+//    FRI tail), whose time is the latency of its own chain. A chain of compressions by one
+//    warp takes 1477 cycles each, against 1640 with every addition on the ALU pipe (a + b + m
+//    as one) and 1960 with every one on the FMA pipe.
+enum AddForm { ADD_FMA, ADD_MIXED };
 
-// a + m[S] + b for a message whose words from W on are zero: no addition for those.
-template <bool FMA, int W, int S>
+// a + b + m[S] (the first or second of a G's two) for a message whose words from W on are
+// zero: no addition for those.
+template <AddForm F, int W, int S, bool SECOND>
 __device__ __forceinline__ uint32_t add_msg(uint32_t a, const uint32_t *m, uint32_t b, uint32_t one) {
-    if constexpr (S < W) return add3<FMA>(a, m[S], b, one);
-    else return add2<FMA>(a, b, one);
+    if constexpr (S >= W) return F == ADD_FMA ? add_on_fma(a, b, one) : a + b;
+    else if constexpr (F == ADD_FMA) return add_on_fma(add_on_fma(a, m[S], one), b, one);
+    else return SECOND ? add_on_fma(a, m[S], one) + b : add_on_fma(a + m[S], b, one);
+}
+template <AddForm F, bool SECOND>
+__device__ __forceinline__ uint32_t add2(uint32_t c, uint32_t d, uint32_t one) {
+    return F == ADD_FMA || SECOND ? add_on_fma(c, d, one) : c + d;
 }
 
-#define STWO_G(a, b, c, d, s, t)          \
-    a = add_msg<FMA, W, s>(a, m, b, one); \
-    d = rotr16(d ^ a);                    \
-    c = add2<FMA>(c, d, one);             \
-    b = rotr(b ^ c, 12);                  \
-    a = add_msg<FMA, W, t>(a, m, b, one); \
-    d = rotr8(d ^ a);                     \
-    c = add2<FMA>(c, d, one);             \
+#define STWO_G(a, b, c, d, s, t)                   \
+    a = add_msg<F, W, s, false>(a, m, b, one);     \
+    d = rotr16(d ^ a);                             \
+    c = add2<F, false>(c, d, one);                 \
+    b = rotr(b ^ c, 12);                           \
+    a = add_msg<F, W, t, true>(a, m, b, one);      \
+    d = rotr8(d ^ a);                              \
+    c = add2<F, true>(c, d, one);                  \
     b = rotr(b ^ c, 7);
 
 // G of the first column step from a zero chaining state (a = b = 0): two additions and two
 // xors fewer.
-#define STWO_G0(a, b, c, d, s, t)         \
-    a = m[s];                             \
-    d = rotr16(d ^ a);                    \
-    c = add2<FMA>(c, d, one);             \
-    b = rotr(c, 12);                      \
-    a = add_msg<FMA, W, t>(a, m, b, one); \
-    d = rotr8(d ^ a);                     \
-    c = add2<FMA>(c, d, one);             \
+#define STWO_G0(a, b, c, d, s, t)                  \
+    a = m[s];                                      \
+    d = rotr16(d ^ a);                             \
+    c = add2<F, false>(c, d, one);                 \
+    b = rotr(c, 12);                               \
+    a = add_msg<F, W, t, true>(a, m, b, one);      \
+    d = rotr8(d ^ a);                              \
+    c = add2<F, true>(c, d, one);                  \
     b = rotr(b ^ c, 7);
 
 // One BLAKE2s round with message permutation s0..s15 (RFC 7693 SIGMA rows).
@@ -103,7 +103,7 @@ __device__ __forceinline__ uint32_t add_msg(uint32_t a, const uint32_t *m, uint3
 // zero (h is only written). X: the two halves of the working state are joined before h is
 // read; the same values, scheduled differently (the tree kernel's 256 x 2^16 trees 89.4 us
 // with it and 91.4 without, the one-layer kernel 686 and 679 us for 64 x 2^22).
-template <bool FMA = true, int W = 16, bool H0 = false, bool X = H0>
+template <AddForm F = ADD_FMA, int W = 16, bool H0 = false, bool X = H0>
 __device__ __forceinline__ void compress_tf(uint32_t h[8], const uint32_t *m, uint32_t t, uint32_t f0, uint32_t one) {
     uint32_t v0 = H0 ? 0u : h[0], v1 = H0 ? 0u : h[1], v2 = H0 ? 0u : h[2], v3 = H0 ? 0u : h[3];
     uint32_t v4 = H0 ? 0u : h[4], v5 = H0 ? 0u : h[5], v6 = H0 ? 0u : h[6], v7 = H0 ? 0u : h[7];
@@ -150,9 +150,9 @@ __device__ __forceinline__ void compress_tf(uint32_t h[8], const uint32_t *m, ui
     h[7] ^= v7 ^ v15;
 }
 
-template <bool FMA = true, int W = 16, bool H0 = false, bool X = H0>
+template <AddForm F = ADD_FMA, int W = 16, bool H0 = false, bool X = H0>
 __device__ __forceinline__ void compress(uint32_t h[8], const uint32_t *m, uint32_t one) {
-    compress_tf<FMA, W, H0, X>(h, m, 0u, 0u, one);
+    compress_tf<F, W, H0, X>(h, m, 0u, 0u, one);
 }
 
 }  // namespace blake

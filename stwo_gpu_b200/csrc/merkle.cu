@@ -172,13 +172,13 @@ __device__ __forceinline__ void merkle_unit(const TreeParams &p, const TreeBand 
                 for (int q = 0; q < 4; q++) {
                     m[4 * q] = v[q].x; m[4 * q + 1] = v[q].y; m[4 * q + 2] = v[q].z; m[4 * q + 3] = v[q].w;
                 }
-                compress<true, 16, true>(h, m, one);
+                compress<blake::ADD_FMA, 16, true>(h, m, one);
             }
             if (nc == 4) {  // a QM31 column: the message's last twelve words are zero
                 uint32_t m4[4];
 #pragma unroll
                 for (int w = 0; w < 4; w++) m4[w] = __ldg(ct[w] + i);
-                compress<true, 4, false, true>(h, m4, one);
+                compress<blake::ADD_FMA, 4, false, true>(h, m4, one);
             } else {
                 // one loop for full chunks and the zero-padded last one (see above)
 #pragma unroll 1
@@ -193,7 +193,7 @@ __device__ __forceinline__ void merkle_unit(const TreeParams &p, const TreeBand 
                             m[w] = cw < nc ? __ldg(ct[cw] + i) : 0u;
                         }
                     }
-                    compress<true, 16, false, true>(h, m, one);
+                    compress<blake::ADD_FMA, 16, false, true>(h, m, one);
                 }
             }
             const uint4 lo = make_uint4(h[0], h[1], h[2], h[3]), hi = make_uint4(h[4], h[5], h[6], h[7]);

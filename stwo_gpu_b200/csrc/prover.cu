@@ -34,6 +34,8 @@
 // u32 words (a bincode-style layout):
 //   commitments, sampled_values, decommitments, queried_values, proof_of_work,
 //   fri_proof{first_layer, inner_layers, last_layer_poly{coeffs, log_size}}.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <chrono>
 #include <cstdlib>
@@ -159,6 +161,19 @@ inline void vanishing_inverses(uint32_t L, uint32_t out[2]) {
     }
 }
 
+// Records a tree's root, mixes it into the channel and draws a felt, with the channel in
+// registers between the two hashes.
+__device__ __forceinline__ qm31 fs_root_step(ProofState *s, const uint32_t *root, uint32_t slot) {
+    fs::DevChannel ch = s->ch;
+    uint32_t r[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) s->roots[slot][i] = r[i] = root[i];
+    fs::ch_mix_root(ch, r);
+    const qm31 v = fs::ch_draw_felt(ch, s->error);
+    s->ch = ch;
+    return v;
+}
+
 // Channel step after the trace tree: mix its root, draw the composition coefficient r,
 // and write powers[k] = r^k (k < n_powers; lane l computes k = l, l + 32, ...).
 __global__ void fs_trace_kernel(ProofState *s, const uint32_t *root, qm31 *powers, uint32_t n_powers, size_t js) {
@@ -168,9 +183,7 @@ __global__ void fs_trace_kernel(ProofState *s, const uint32_t *root, qm31 *power
     powers = job_ptr(powers, js, blockIdx.x);
     __shared__ qm31 rc;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 8; i++) s->roots[0][i] = root[i];
-        fs::ch_mix_root(s->ch, root);
-        rc = fs::ch_draw_felt(s->ch, s->error);
+        rc = fs_root_step(s, root, 0);
         s->rc = rc;
     }
     __syncthreads();
@@ -189,9 +202,7 @@ __global__ void fs_comp_kernel(ProofState *s, const uint32_t *root, size_t js) {
     chain_wait();
     s = job_ptr(s, js, blockIdx.x);  // one thread a job
     root = job_ptr(root, js, blockIdx.x);
-    for (int i = 0; i < 8; i++) s->roots[1][i] = root[i];
-    fs::ch_mix_root(s->ch, root);
-    const qm31 t = fs::ch_draw_felt(s->ch, s->error), t2 = qm31_mul(t, t);
+    const qm31 t = fs_root_step(s, root, 1), t2 = qm31_mul(t, t);
     const qm31 inv = qm31_inv(qm31_add(t2, qm31_one()));
     s->oods[0] = qm31_mul(qm31_sub(qm31_one(), t2), inv);
     s->oods[1] = qm31_mul(qm31_add(t, t), inv);
@@ -265,9 +276,7 @@ __global__ void fs_layer_kernel(ProofState *s, const uint32_t *root, uint32_t ro
     chain_wait();
     s = job_ptr(s, js, blockIdx.x);  // one thread a job
     root = job_ptr(root, js, blockIdx.x);
-    for (int i = 0; i < 8; i++) s->roots[root_slot][i] = root[i];
-    fs::ch_mix_root(s->ch, root);
-    s->alphas[alpha_slot] = fs::ch_draw_felt(s->ch, s->error);
+    s->alphas[alpha_slot] = fs_root_step(s, root, root_slot);
 }
 
 // Last FRI layer: 2^log values (bit-reversed) over the line domain
@@ -298,23 +307,33 @@ __device__ void fs_last(ProofState *s, const uint32_t *const c[4], uint32_t log)
     fs::ch_mix_felts(s->ch, &c0, 1);
 }
 
-// The FRI tail in one launch: one CTA of 1024 threads runs every inner layer of log
-// size <= TAIL_MAX_LOG in order, then the last layer, exactly as the per-layer
-// launches do:
+// The FRI tail in one launch: one cluster of eight CTAs runs every inner layer of log size
+// <= TAIL_MAX_LOG in order, then the last layer, exactly as the per-layer launches do:
 //   [the trace quotient's circle fold into the layer, with the previous alpha]
 //   -> the layer's Merkle tree over its 4 coordinate columns (leaves: one compression
 //      of the 4 values; nodes: one compression of the two children), every level
 //      written to its global buffer for the decommitment and kept in shared memory
 //      for the next level
-//   -> thread 0: mix the root, draw the layer's alpha
+//   -> thread 0 of CTA 0: mix the root, draw the layer's alpha
 //   -> fold_line into the next layer.
+// The chain of tree levels and channel steps is serial (about 1900 cycles a level), so the
+// cluster only spreads the wide levels: in layers of log size >= TAIL_SPLIT_LOG each CTA
+// owns an eighth of the values and of every level down to eight nodes, which CTA 0 reads
+// through distributed shared memory and finishes; alpha goes back the same way. A CTA's folded
+// values are its own eighth of the next layer. Smaller layers are CTA 0's alone. (One CTA of
+// 1024 threads hashed the 1024 leaves of log size 10 in 12.8k cycles, and log sizes 11 to 13
+// took three launches a layer: a 64-column x 2^12 proof FIGURES.)
 // Values this kernel wrote are read back with plain (coherent) loads after a
 // barrier; nothing is read through the non-coherent path except the trace quotient
 // and the twiddles.
-constexpr uint32_t TAIL_MAX_LOG = 10;
+constexpr uint32_t TAIL_MAX_LOG = 13;
 constexpr uint32_t TAIL_MAX = TAIL_MAX_LOG;  // inner layers of log size 2 .. TAIL_MAX_LOG
-constexpr uint32_t TAIL_THREADS = 1024;
-constexpr size_t TAIL_SMEM = (32ull << TAIL_MAX_LOG) + (32ull << (TAIL_MAX_LOG - 1));
+constexpr uint32_t TAIL_CTAS_LOG = 3, TAIL_CTAS = 1u << TAIL_CTAS_LOG;
+constexpr uint32_t TAIL_SPLIT_LOG = 9;
+constexpr uint32_t TAIL_THREADS = 256;
+constexpr uint32_t TAIL_LOCAL_LOG = TAIL_MAX_LOG - TAIL_CTAS_LOG;  // a CTA's leaves of the largest layer
+constexpr size_t TAIL_SMEM = (32ull << TAIL_LOCAL_LOG) + (32ull << (TAIL_LOCAL_LOG - 1));
+static_assert(TAIL_SPLIT_LOG <= TAIL_LOCAL_LOG + 1, "a layer of CTA 0's alone fits its node buffers");
 
 struct TailParams {
     uint32_t li0, n_tail, lg0, last_log;
@@ -326,23 +345,32 @@ struct TailParams {
     const uint32_t *line_tw[TAIL_MAX];            // inverse-twiddle suffix of each layer's line fold
 };
 
-__global__ void __launch_bounds__(TAIL_THREADS) fri_tail_kernel(ProofState *s, const TailParams *__restrict__ tp,
-                                                                 uint32_t one, size_t js) {
+__global__ void __cluster_dims__(TAIL_CTAS, 1, 1) __launch_bounds__(TAIL_THREADS)
+    fri_tail_kernel(ProofState *s, const TailParams *__restrict__ tp, uint32_t one, size_t js) {
     chain_wait();
-    s = job_ptr(s, js, blockIdx.x);  // one CTA a job; the job's parameters hold its own pointers
-    tp = job_ptr(tp, js, blockIdx.x);
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t rank = cluster.block_rank(), job = blockIdx.x / TAIL_CTAS;
+    s = job_ptr(s, js, job);  // one cluster a job; the job's parameters hold its own pointers
+    tp = job_ptr(tp, js, job);
     extern __shared__ uint4 t_buf[];
     // the two node buffers, by computed address (an indexed pointer array would live
     // in local memory)
-    auto buf = [&](uint32_t which) { return t_buf + (which ? (2u << TAIL_MAX_LOG) : 0u); };
+    auto buf = [&](uint32_t which) { return t_buf + (which ? (2u << TAIL_LOCAL_LOG) : 0u); };
     __shared__ qm31 alpha_sh;
     const uint32_t tid = threadIdx.x;
+    fs::DevChannel ch;  // thread 0 of CTA 0 keeps the channel in registers
+    if (rank == 0 && tid == 0) ch = s->ch;
     for (uint32_t t = 0; t < tp->n_tail; t++) {
-        const uint32_t li = tp->li0 + t, lg = tp->lg0 - t, n = 1u << lg;
+        const uint32_t li = tp->li0 + t, lg = tp->lg0 - t;
+        const bool split = lg >= TAIL_SPLIT_LOG;
+        if (!split && rank != 0) return;  // (the fold into this layer ended with a cluster barrier)
+        // this CTA's values of the layer
+        const uint32_t n = split ? 1u << (lg - TAIL_CTAS_LOG) : 1u << lg, first = split ? rank * n : 0u;
         uint32_t *const *cur = tp->lay[t];
         if (t == tp->circle_t) {
-            const qm31 a = s->alphas[li], a2 = qm31_mul(a, a);
-            for (uint32_t i = tid; i < n; i += TAIL_THREADS) {
+            const qm31 a = t == 0 ? s->alphas[li] : alpha_sh, a2 = qm31_mul(a, a);
+            for (uint32_t i = first + tid; i < first + n; i += TAIL_THREADS) {
                 const qm31 f0 = {{__ldg(tp->qt[0] + 2 * i), __ldg(tp->qt[1] + 2 * i)},
                                  {__ldg(tp->qt[2] + 2 * i), __ldg(tp->qt[3] + 2 * i)}};
                 const qm31 f1 = {{__ldg(tp->qt[0] + 2 * i + 1), __ldg(tp->qt[1] + 2 * i + 1)},
@@ -358,21 +386,22 @@ __global__ void __launch_bounds__(TAIL_THREADS) fri_tail_kernel(ProofState *s, c
             __syncthreads();
         }
         // Leaves: one compression of the layer's 4 values.
-        for (uint32_t i = tid; i < n; i += TAIL_THREADS) {
+        for (uint32_t k = tid; k < n; k += TAIL_THREADS) {
+            const uint32_t i = first + k;
             uint32_t h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
             uint32_t m[16] = {cur[0][i], cur[1][i], cur[2][i], cur[3][i], 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-            blake::compress(h, m, one);
+            blake::compress<blake::ADD_MIXED>(h, m, one);
             const uint4 lo = make_uint4(h[0], h[1], h[2], h[3]), hi = make_uint4(h[4], h[5], h[6], h[7]);
             tp->nodes[t][lg][2 * i] = lo;
             tp->nodes[t][lg][2 * i + 1] = hi;
-            buf(0)[2 * i] = lo;
-            buf(0)[2 * i + 1] = hi;
+            buf(0)[2 * k] = lo;
+            buf(0)[2 * k + 1] = hi;
         }
         __syncthreads();
-        // Nodes, level by level: children from one shared buffer, parents into the other.
-        // Levels of at most 32 nodes are left to the first warp, which synchronises
-        // with itself only.
-        auto node = [&](uint32_t l, uint32_t k, uint32_t src) {
+        // Nodes, level by level: children from one shared buffer, parents into the other. `at`
+        // is the CTA's first node of the level. Levels of at most 32 nodes are left to the first
+        // warp, which synchronises with itself only.
+        auto node = [&](uint32_t l, uint32_t at, uint32_t k, uint32_t src) {
             uint32_t h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
             uint32_t m[16];
 #pragma unroll
@@ -380,41 +409,61 @@ __global__ void __launch_bounds__(TAIL_THREADS) fri_tail_kernel(ProofState *s, c
                 const uint4 v = buf(src)[4 * k + q];
                 m[4 * q] = v.x; m[4 * q + 1] = v.y; m[4 * q + 2] = v.z; m[4 * q + 3] = v.w;
             }
-            blake::compress(h, m, one);
+            blake::compress<blake::ADD_MIXED>(h, m, one);
             const uint4 lo = make_uint4(h[0], h[1], h[2], h[3]), hi = make_uint4(h[4], h[5], h[6], h[7]);
-            tp->nodes[t][l][2 * k] = lo;
-            tp->nodes[t][l][2 * k + 1] = hi;
+            tp->nodes[t][l][2 * (at + k)] = lo;
+            tp->nodes[t][l][2 * (at + k) + 1] = hi;
             buf(src ^ 1)[2 * k] = lo;
             buf(src ^ 1)[2 * k + 1] = hi;
         };
-        uint32_t src = 0;
+        uint32_t src = 0, count = n >> 1;
         int l = (int)lg - 1;
-        for (; l >= 0 && (1u << l) > 32u; l--) {
-            for (uint32_t k = tid; k < (1u << l); k += TAIL_THREADS) node((uint32_t)l, k, src);
+        for (; count > 32u; l--, count >>= 1) {
+            for (uint32_t k = tid; k < count; k += TAIL_THREADS) node((uint32_t)l, split ? rank * count : 0u, k, src);
             src ^= 1;
             __syncthreads();
         }
-        if (tid < 32) {  // src is only read by thread 0 below
-            for (; l >= 0; l--) {
-                if (tid < (1u << l)) node((uint32_t)l, tid, src);
-                src ^= 1;
+        // The first warp's levels, in a split layer in two runs: down to the CTA's one node,
+        // then, in CTA 0, from the cluster's eight.
+        for (bool gathered = !split;; gathered = true) {
+            if (tid < 32) {
+                for (; count > 0; l--, count >>= 1) {
+                    if (tid < count) node((uint32_t)l, gathered ? 0u : rank * count, tid, src);
+                    src ^= 1;
+                    __syncwarp();
+                }
+            }
+            if (gathered) break;
+            cluster.sync();  // every CTA's node is in its buffer
+            if (rank == 0) {
+                if (tid < TAIL_CTAS) {
+                    const uint4 *theirs = cluster.map_shared_rank(buf(src), tid);
+                    const uint4 lo = theirs[0], hi = theirs[1];
+                    __syncwarp((1u << TAIL_CTAS) - 1u);
+                    buf(src)[2 * tid] = lo;
+                    buf(src)[2 * tid + 1] = hi;
+                }
                 __syncwarp();
+                count = TAIL_CTAS / 2;
             }
         }
-        if (tid == 0) {
+        if (rank == 0 && tid == 0) {  // (src is only right in the first warp)
             const uint4 lo = buf(src)[0], hi = buf(src)[1];
             const uint32_t root[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
             for (int i = 0; i < 8; i++) s->roots[3 + li][i] = root[i];
-            fs::ch_mix_root(s->ch, root);
-            const qm31 a = fs::ch_draw_felt(s->ch, s->error);
+            fs::ch_mix_root(ch, root);
+            const qm31 a = fs::ch_draw_felt(ch, s->error);
             s->alphas[li + 1] = a;
             alpha_sh = a;
+            if (split)
+                for (uint32_t r = 1; r < TAIL_CTAS; r++) *cluster.map_shared_rank(&alpha_sh, r) = a;
         }
-        __syncthreads();
+        if (split) cluster.sync();
+        else __syncthreads();
         // fold_line into the next layer.
         const qm31 alpha = alpha_sh;
         uint32_t *const *nxt = tp->lay[t + 1];
-        for (uint32_t i = tid; i < n / 2; i += TAIL_THREADS) {
+        for (uint32_t i = first / 2 + tid; i < (first + n) / 2; i += TAIL_THREADS) {
             const qm31 f0 = {{cur[0][2 * i], cur[1][2 * i]}, {cur[2][2 * i], cur[3][2 * i]}};
             const qm31 f1 = {{cur[0][2 * i + 1], cur[1][2 * i + 1]}, {cur[2][2 * i + 1], cur[3][2 * i + 1]}};
             const qm31 r = fold_pair(f0, f1, __ldg(tp->line_tw[t] + i), alpha);
@@ -423,9 +472,14 @@ __global__ void __launch_bounds__(TAIL_THREADS) fri_tail_kernel(ProofState *s, c
             nxt[2][i] = r.b.a;
             nxt[3][i] = r.b.b;
         }
-        __syncthreads();
+        // before CTA 0 goes on alone it needs every CTA's values
+        if (split && lg == TAIL_SPLIT_LOG) cluster.sync();
+        else __syncthreads();
     }
-    if (tid == 0) fs_last(s, tp->lay[tp->n_tail], tp->last_log);
+    if (rank == 0 && tid == 0) {
+        s->ch = ch;
+        fs_last(s, tp->lay[tp->n_tail], tp->last_log);
+    }
 }
 
 int launch_fri_tail(ProofState *s, const TailParams *tp, uint32_t jobs, size_t js, cudaStream_t st) {
@@ -435,7 +489,7 @@ int launch_fri_tail(ProofState *s, const TailParams *tp, uint32_t jobs, size_t j
         return (int)STWO_OK;
     });
     if (rc) return rc;
-    launch_chained(fri_tail_kernel, jobs, TAIL_THREADS, TAIL_SMEM, st, s, tp, 1u, js);
+    launch_chained(fri_tail_kernel, jobs * TAIL_CTAS, TAIL_THREADS, TAIL_SMEM, st, s, tp, 1u, js);
     STWO_LAUNCH_CHECK("fri_tail_kernel");
     return STWO_OK;
 }
@@ -488,12 +542,14 @@ __global__ void fs_finish_kernel(ProofState *s, uint32_t n_queries, size_t js) {
         s->error |= fs::ERR_GRIND;
         return;
     }
-    fs::ch_mix_nonce(s->ch, s->nonce);
+    fs::DevChannel ch = s->ch;
+    fs::ch_mix_nonce(ch, s->nonce);
     for (uint32_t q = 0; q < n_queries; q += 8) {
         uint32_t w[8];
-        fs::ch_draw_words(s->ch, w);
+        fs::ch_draw_words(ch, w);
         for (uint32_t i = 0; i < 8 && q + i < n_queries; i++) s->query_words[q + i] = w[i];
     }
+    s->ch = ch;
 }
 
 // Reads of single words from device buffers (decommitment values and witnesses).
