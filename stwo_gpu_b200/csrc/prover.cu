@@ -40,10 +40,8 @@
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
-#include <map>
 #include <memory>
 #include <new>
-#include <set>
 #include <vector>
 
 #include "blake2s.cuh"
@@ -552,16 +550,20 @@ __global__ void fs_finish_kernel(ProofState *s, uint32_t n_queries, size_t js) {
     s->ch = ch;
 }
 
-// Reads of single words from device buffers (decommitment values and witnesses).
+// Reads of runs of up to eight words from device buffers (decommitment values and witnesses).
+// The requests are read from pinned host memory and the words written there, without a copy
+// either way; eight threads a request.
 struct GatherReq {
-    const uint32_t *ptr;
-    uint64_t idx;
+    const uint32_t *src;
+    uint32_t words, out;  // out: index of the first word in the output
 };
 
 __global__ void gather_kernel(const GatherReq *__restrict__ req, uint32_t n, uint32_t *__restrict__ out) {
     chain_wait();
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = req[i].ptr[req[i].idx];
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, i = t >> 3, w = t & 7u;
+    if (i >= n) return;
+    const GatherReq r = req[i];
+    if (w < r.words) out[r.out + w] = r.src[w];
 }
 
 // ------------------------------------------------------------------ host plumbing
@@ -681,32 +683,39 @@ int plan_tree(MerkleTree &t, std::vector<std::pair<uint32_t, const uint32_t *>> 
     return STWO_OK;
 }
 
-// Word reads from device memory, planned on the host and executed in one launch.
+// Reads from device memory, planned on the host and executed in one launch: each request's
+// words follow those of the request before, so values that are written to the proof in a row
+// are requested in a row.
 struct Gatherer {
     std::vector<GatherReq> reqs;
-    std::vector<uint32_t> vals;
-    size_t add(const uint32_t *p, uint64_t idx) {
-        reqs.push_back({p, idx});
-        return reqs.size() - 1;
+    uint32_t n_words = 0;
+    const uint32_t *vals = nullptr;  // after run(), until the thread's next host_stage
+    uint32_t add(const uint32_t *src, uint32_t words) {
+        const uint32_t at = n_words;
+        reqs.push_back({src, words, at});
+        n_words += words;
+        return at;
     }
-    int run(Arena &ar, cudaStream_t st) {
-        vals.assign(reqs.size(), 0);
+    int run(cudaStream_t st) {
         if (reqs.empty()) return STWO_OK;
-        PV_ALLOC(dreq, GatherReq, reqs.size());
-        PV_ALLOC(dout, uint32_t, reqs.size());
+        STWO_REQUIRE(reqs.size() < (1u << 28), STWO_ERR_UNSUPPORTED_SIZE, "decommitment of %zu reads", reqs.size());
         const size_t req_bytes = reqs.size() * sizeof(GatherReq);
         void *stage = nullptr;
-        PV_TRY(host_stage(req_bytes + reqs.size() * 4, &stage));
+        PV_TRY(host_stage(req_bytes + (size_t)n_words * 4, &stage));
         memcpy(stage, reqs.data(), req_bytes);
-        uint32_t *out_stage = reinterpret_cast<uint32_t *>(static_cast<uint8_t *>(stage) + req_bytes);
-        STWO_CUDA_TRY(cudaMemcpyAsync(dreq, stage, req_bytes, cudaMemcpyHostToDevice, st));
-        launch_chained(gather_kernel, (unsigned)((reqs.size() + 255) / 256), 256, 0, st, dreq, (uint32_t)reqs.size(), dout);
+        uint32_t *out = reinterpret_cast<uint32_t *>(static_cast<uint8_t *>(stage) + req_bytes);
+        launch_chained(gather_kernel, (unsigned)((reqs.size() * 8 + 255) / 256), 256, 0, st,
+                       static_cast<const GatherReq *>(stage), (uint32_t)reqs.size(), out);
         STWO_LAUNCH_CHECK("gather_kernel");
-        STWO_CUDA_TRY(cudaMemcpyAsync(out_stage, dout, reqs.size() * 4, cudaMemcpyDeviceToHost, st));
         PV_TRY(wait_stream(st));
-        memcpy(vals.data(), out_stage, reqs.size() * 4);
+        vals = out;
         return STWO_OK;
     }
+};
+
+// Values of one kind in the gathered words: `count` items from `first` on.
+struct Gathered {
+    uint32_t first = 0, count = 0;
 };
 
 // MerkleProver::decommit, planned: layer by layer from the leaves, the nodes to open
@@ -715,63 +724,84 @@ struct Gatherer {
 // opened node are queried values when the node is a queried position, else column
 // witness.
 struct TreeDecommit {
-    std::vector<size_t> hash_words;            // 8 gather indices per witness hash
-    std::vector<size_t> column_witness;        // gather indices
-    std::vector<std::vector<size_t>> queried;  // per column (tree order), gather indices
+    Gathered hashes;                // 8 words each
+    Gathered column_witness;        // words
+    std::vector<Gathered> queried;  // per column (tree order), words
 };
 
-TreeDecommit plan_decommit(const MerkleTree &t, const std::map<uint32_t, std::vector<uint64_t>> &queries,
-                           Gatherer &g) {
+// Queried positions of the columns of one log size, ascending.
+using LogQueries = std::pair<uint32_t, std::vector<uint64_t>>;
+
+TreeDecommit plan_decommit(const MerkleTree &t, std::initializer_list<const LogQueries *> queries, Gatherer &g) {
+    static const std::vector<uint64_t> none;
+    struct Layer {
+        size_t col0, col1;  // its columns
+        const std::vector<uint64_t> *colq;
+        std::vector<uint64_t> witness;  // opened nodes that are no queried position
+    };
     TreeDecommit d;
-    d.queried.assign(t.cols.size(), {});
-    std::vector<uint64_t> below;  // opened nodes of the layer below, sorted
+    d.queried.resize(t.cols.size());
+    std::vector<Layer> layers;
+    std::vector<uint64_t> below, nodes;  // opened nodes of the layer below and of this one, ascending
+    size_t col = 0;
+    d.hashes.first = g.n_words;
     for (int l = (int)t.max_log; l >= 0; l--) {
-        std::vector<size_t> lc;
-        for (size_t i = 0; i < t.cols.size(); i++)
-            if (t.cols[i].first == (uint32_t)l) lc.push_back(i);
-        std::set<uint64_t> colq;
-        auto it = queries.find((uint32_t)l);
-        if (it != queries.end()) colq.insert(it->second.begin(), it->second.end());
-        std::set<uint64_t> nodes(colq);
-        for (uint64_t q : below) nodes.insert(q >> 1);
-        const std::set<uint64_t> opened_below(below.begin(), below.end());
-        for (uint64_t node : nodes) {
-            if (l < (int)t.max_log) {
-                for (uint64_t child : {2 * node, 2 * node + 1})
-                    if (!opened_below.count(child))
-                        for (int w = 0; w < 8; w++) d.hash_words.push_back(g.add(t.layers[l + 1], child * 8 + w));
-            }
-            const bool queried = colq.count(node) > 0;
-            for (size_t ci : lc) {
-                size_t gi = g.add(t.cols[ci].second, node);
-                if (queried) d.queried[ci].push_back(gi);
-                else d.column_witness.push_back(gi);
-            }
+        Layer y{col, col, &none, {}};
+        while (y.col1 < t.cols.size() && t.cols[y.col1].first == (uint32_t)l) y.col1++;
+        col = y.col1;
+        for (const LogQueries *q : queries)
+            if (q->first == (uint32_t)l) y.colq = &q->second;
+        // nodes: the merge of the queried positions and the parents
+        nodes.clear();
+        size_t iq = 0, ib = 0;
+        while (iq < y.colq->size() || ib < below.size()) {
+            const uint64_t a = iq < y.colq->size() ? (*y.colq)[iq] : ~0ull, b = ib < below.size() ? below[ib] >> 1 : ~0ull;
+            const uint64_t node = std::min(a, b);
+            nodes.push_back(node);
+            if (a == node) iq++;
+            else if (y.col1 > y.col0) y.witness.push_back(node);
+            bool open[2] = {false, false};
+            for (; ib < below.size() && below[ib] >> 1 == node; ib++) open[below[ib] & 1] = true;
+            if (l < (int)t.max_log)
+                for (uint64_t c = 0; c < 2; c++)
+                    if (!open[c]) {
+                        g.add(t.layers[l + 1] + (2 * node + c) * 8, 8);
+                        d.hashes.count++;
+                    }
         }
-        below.assign(nodes.begin(), nodes.end());
+        if (y.col1 > y.col0) layers.push_back(std::move(y));
+        below.swap(nodes);
     }
+    d.column_witness.first = g.n_words;
+    for (const Layer &y : layers)
+        for (uint64_t node : y.witness)
+            for (size_t c = y.col0; c < y.col1; c++) g.add(t.cols[c].second + node, 1);
+    d.column_witness.count = g.n_words - d.column_witness.first;
+    for (const Layer &y : layers)
+        for (size_t c = y.col0; c < y.col1; c++) {
+            d.queried[c] = {g.n_words, (uint32_t)y.colq->size()};
+            for (uint64_t node : *y.colq) g.add(t.cols[c].second + node, 1);
+        }
     return d;
 }
 
 // Proof byte stream.
 struct Writer {
     std::vector<uint8_t> b;
-    void u32(uint32_t v) { b.insert(b.end(), (uint8_t *)&v, (uint8_t *)&v + 4); }
-    void u64(uint64_t v) { b.insert(b.end(), (uint8_t *)&v, (uint8_t *)&v + 8); }
     void bytes(const void *p, size_t n) { b.insert(b.end(), (const uint8_t *)p, (const uint8_t *)p + n); }
+    void u32(uint32_t v) { bytes(&v, 4); }
+    void u64(uint64_t v) { bytes(&v, 8); }
     void q(qm31 v) {
-        u32(v.a.a);
-        u32(v.a.b);
-        u32(v.b.a);
-        u32(v.b.b);
+        const uint32_t w[4] = {v.a.a, v.a.b, v.b.a, v.b.b};
+        bytes(w, 16);
     }
 };
 
-void write_decommitment(Writer &w, const TreeDecommit &d, const std::vector<uint32_t> &vals) {
-    w.u64(d.hash_words.size() / 8);
-    for (size_t gi : d.hash_words) w.u32(vals[gi]);
-    w.u64(d.column_witness.size());
-    for (size_t gi : d.column_witness) w.u32(vals[gi]);
+void write_decommitment(Writer &w, const TreeDecommit &d, const uint32_t *vals) {
+    w.u64(d.hashes.count);
+    w.bytes(vals + d.hashes.first, (size_t)d.hashes.count * 32);
+    w.u64(d.column_witness.count);
+    w.bytes(vals + d.column_witness.first, (size_t)d.column_witness.count * 4);
 }
 
 std::vector<uint64_t> fold_queries(const std::vector<uint64_t> &q, uint32_t n) {
@@ -1155,7 +1185,7 @@ int prove_jobs(const Job &j, uint32_t K, const uint32_t *const *a0_in, const uin
                          "a job of the batch does not fit its slab");
             ar.bytes += sub.bytes;
         }
-        ar.used = ar.cap;  // the jobs' slabs are taken: later allocations (the gather) go past them
+        ar.used = ar.cap;  // the jobs' slabs are taken
     }
     JobLayout &J = jl[0];
     const uint32_t *tw = J.tw, *itw = J.itw;
@@ -1375,8 +1405,8 @@ int prove_jobs(const Job &j, uint32_t K, const uint32_t *const *a0_in, const uin
     struct JobDecommit {
         int rc = STWO_OK;
         TreeDecommit d_trace, d_comp, d_fri0;
-        std::vector<size_t> w_first;
-        std::vector<std::vector<size_t>> w_inner;
+        Gathered w_first;               // QM31 values
+        std::vector<Gathered> w_inner;
         std::vector<TreeDecommit> d_inner;
     };
     std::vector<JobDecommit> jd(K);
@@ -1393,45 +1423,50 @@ int prove_jobs(const Job &j, uint32_t K, const uint32_t *const *a0_in, const uin
         // Queries::generate over the largest quotient domain (log D).
         std::vector<uint64_t> queries;
         {
-            std::set<uint64_t> qs;
             const uint32_t mask = (uint32_t)((1ull << D) - 1);
-            for (uint32_t i = 0; i < j.n_queries; i++) qs.insert(ps.query_words[i] & mask);
-            queries.assign(qs.begin(), qs.end());
+            for (uint32_t i = 0; i < j.n_queries; i++) queries.push_back(ps.query_words[i] & mask);
+            std::sort(queries.begin(), queries.end());
+            queries.erase(std::unique(queries.begin(), queries.end()), queries.end());
         }
-        const std::map<uint32_t, std::vector<uint64_t>> tree_queries = {{D, queries},
-                                                                        {L + B, fold_queries(queries, 1)}};
-        o.d_trace = plan_decommit(Jk.t_trace, tree_queries, g);
-        o.d_comp = plan_decommit(Jk.t_comp, tree_queries, g);
+        // The values of `at` of a secure column, consecutive in the gathered words.
+        auto gather_qm31 = [&](const std::vector<uint32_t *> &col, const std::vector<uint64_t> &at, Gathered &out) {
+            out.count += (uint32_t)at.size();
+            for (uint64_t x : at)
+                for (int c = 0; c < 4; c++) g.add(col[c] + x, 1);
+        };
+        const LogQueries q_comp{D, queries}, q_trace{L + B, fold_queries(queries, 1)};
+        o.d_trace = plan_decommit(Jk.t_trace, {&q_trace}, g);
+        o.d_comp = plan_decommit(Jk.t_comp, {&q_comp}, g);
         // FRI first layer: per quotient column, its folding pairs; partners are witnesses.
         {
-            std::map<uint32_t, std::vector<uint64_t>> pos;
+            LogQueries pos[2];
+            o.w_first.first = g.n_words;
             for (int grp = 0; grp < 2; grp++) {
                 const uint32_t lg = grp == 0 ? D : L + B;
-                const std::vector<uint32_t *> &col = grp == 0 ? Jk.qc : Jk.qt;
-                std::vector<uint64_t> p, wv;
-                fri_positions(fold_queries(queries, D - lg), p, wv);
-                pos[lg] = p;
-                for (uint64_t x : wv)
-                    for (int c = 0; c < 4; c++) o.w_first.push_back(g.add(col[c], x));
+                std::vector<uint64_t> wv;
+                pos[grp].first = lg;
+                fri_positions(fold_queries(queries, D - lg), pos[grp].second, wv);
+                gather_qm31(grp == 0 ? Jk.qc : Jk.qt, wv, o.w_first);
             }
-            o.d_fri0 = plan_decommit(Jk.t_fri0, pos, g);
+            o.d_fri0 = plan_decommit(Jk.t_fri0, {&pos[0], &pos[1]}, g);
         }
-        o.w_inner.assign(n_layers, {});
-        o.d_inner.assign(n_layers, {});
+        o.w_inner.resize(n_layers);
+        o.d_inner.resize(n_layers);
         {
             std::vector<uint64_t> lq = fold_queries(queries, 1);
             for (uint32_t li = 0; li < n_layers; li++) {
-                std::vector<uint64_t> p, wv;
-                fri_positions(lq, p, wv);
-                for (uint64_t x : wv)
-                    for (int c = 0; c < 4; c++) o.w_inner[li].push_back(g.add(Jk.lay[li][c], x));
-                o.d_inner[li] = plan_decommit(Jk.t_lay[li], {{D - 1 - li, p}}, g);
+                LogQueries pos{D - 1 - li, {}};
+                std::vector<uint64_t> wv;
+                fri_positions(lq, pos.second, wv);
+                o.w_inner[li].first = g.n_words;
+                gather_qm31(Jk.lay[li], wv, o.w_inner[li]);
+                o.d_inner[li] = plan_decommit(Jk.t_lay[li], {&pos}, g);
                 lq = fold_queries(lq, 1);
             }
         }
     }
-    PV_TRY(g.run(ar, st));
-    const std::vector<uint32_t> &vals = g.vals;
+    PV_TRY(g.run(st));
+    const uint32_t *vals = g.vals;
 
     // ---- serialisation
     uint64_t proof_bytes = 0;
@@ -1445,6 +1480,7 @@ int prove_jobs(const Job &j, uint32_t K, const uint32_t *const *a0_in, const uin
         const ProofState &ps = *reinterpret_cast<const ProofState *>(rec.data() + rec_bytes * k);
         const qm31 *sampled = reinterpret_cast<const qm31 *>(rec.data() + rec_bytes * k + sizeof(ProofState));
         Writer w;
+        w.b.reserve(4096 + 32ull * (N + 4) + 64ull * (n_layers + 3) + 4ull * g.n_words / K);
         w.u64(2);  // commitments
         w.bytes(ps.roots[0], 32);
         w.bytes(ps.roots[1], 32);
@@ -1465,15 +1501,15 @@ int prove_jobs(const Job &j, uint32_t K, const uint32_t *const *a0_in, const uin
         w.u64(2);  // queried_values
         for (const TreeDecommit *d : {&o.d_trace, &o.d_comp}) {
             w.u64(d->queried.size());
-            for (auto &col : d->queried) {
-                w.u64(col.size());
-                for (size_t gi : col) w.u32(vals[gi]);
+            for (const Gathered &col : d->queried) {
+                w.u64(col.count);
+                w.bytes(vals + col.first, (size_t)col.count * 4);
             }
         }
         w.u64(ps.nonce);  // proof_of_work
-        auto write_fri_layer = [&](const std::vector<size_t> &wit, const TreeDecommit &d, const uint32_t root[8]) {
-            w.u64(wit.size() / 4);
-            for (size_t gi : wit) w.u32(vals[gi]);
+        auto write_fri_layer = [&](const Gathered &wit, const TreeDecommit &d, const uint32_t root[8]) {
+            w.u64(wit.count);
+            w.bytes(vals + wit.first, (size_t)wit.count * 16);
             write_decommitment(w, d, vals);
             w.bytes(root, 32);
         };
