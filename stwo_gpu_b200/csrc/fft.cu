@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(1 << MAX_THREADS_LOG) fft_pass_kernel(const __
 // back (their twiddles are then L2 hits); strided passes run the 2^(N-hi) copies of
 // an extension read back to back (the coefficient tile is then an L2 hit).
 // ---------------------------------------------------------------------------
-constexpr int TT = 14;  // tile = 2^14 elements; a thread owns 2^E of them (E = 5 or 6)
+constexpr int TT = 14;  // tile = 2^T elements, T = TT but for the small launches of launchT_t; 2^E a thread
 
 __host__ __device__ constexpr uint32_t swz_c(uint32_t j) { return j ^ (((j >> 5) ^ (j >> 10)) & 31u); }
 
@@ -265,16 +265,16 @@ __host__ __device__ constexpr uint32_t bank_vec(int b) {
     return (b < 5 ? 1u << b : 0u) ^ (b >= 5 && b < 10 ? 1u << (b - 5) : 0u) ^ (b >= 10 && b < 15 ? 1u << (b - 10) : 0u);
 }
 
-struct BitMap { int pos[TT]; };
+struct BitMap { int pos[TT]; };  // (a tile of 2^T elements uses the first T)
 
 // Positions (tile bits) of the thread-index bits of a round owning [OA, OA+RB):
 // lanes first (the lowest other bits, or for middle rounds the lowest bits with
 // independent bank images), then the remaining other bits in increasing order.
-__host__ __device__ constexpr BitMap make_map(int OA, int RB, bool pick_lanes) {
+__host__ __device__ constexpr BitMap make_map(int T, int OA, int RB, bool pick_lanes) {
     BitMap m{};
     int other[TT] = {};
     int n = 0;
-    for (int b = 0; b < TT; b++)
+    for (int b = 0; b < T; b++)
         if (b < OA || b >= OA + RB) other[n++] = b;
     bool used[TT] = {};
     int k = 0;
@@ -323,10 +323,10 @@ struct GeoT {
 };
 
 // Global index of tile element jb within its column.
-template <int G, int C, int LO>
+template <int G, int C, int LO, int T>
 __device__ __forceinline__ uint32_t tile_index(const GeoT &geo, uint32_t jb) {
     if constexpr (C == 0) {
-        if constexpr (G == TT) return geo.gfix | jb;
+        if constexpr (G == T) return geo.gfix | jb;
         else return geo.gfix | (jb & ((1u << geo.nc) - 1u));
     } else {
         const uint32_t lo = LO ? (uint32_t)LO : geo.p->lo;
@@ -336,12 +336,12 @@ __device__ __forceinline__ uint32_t tile_index(const GeoT &geo, uint32_t jb) {
 
 // Source and destination of the column that tile element jb belongs to; false when the
 // launch has no such column (the last tile of a launch of short columns).
-template <int G, int C>
+template <int G, int C, int T>
 __device__ __forceinline__ bool tile_column(const GeoT &geo, uint32_t jb, const uint32_t *&src, uint32_t *&dst) {
     src = geo.src;
     dst = geo.dst;
-    if constexpr (C == 0 && G < TT) {
-        if (geo.nc < (uint32_t)TT) {
+    if constexpr (C == 0 && G < T) {
+        if (geo.nc < (uint32_t)T) {
             const uint32_t col = geo.col + (jb >> geo.nc);
             if (col >= geo.n_cols) return false;
             const FftColumn fc = fft_col(*geo.p, col);
@@ -452,15 +452,15 @@ __device__ __forceinline__ uint32_t turn_slot(uint32_t r, uint32_t c) {
     return (r << LCH) + (c ^ f);
 }
 
-template <int G, int C, bool INV, int R, int E, int LO>
+template <int G, int C, bool INV, int R, int E, int LO, int T>
 __device__ __forceinline__ void roundT(uint32_t *sm, const GeoT &geo) {
     using RI = RoundT<G, INV, R, E>;
-    constexpr int RB = RI::RB, A = RI::A, OA = C + A, RR = 1 << RB, GROUPS = 1 << (E - RB), W = TT - E;
+    constexpr int RB = RI::RB, A = RI::A, OA = C + A, RR = 1 << RB, GROUPS = 1 << (E - RB), W = T - E;
     constexpr bool FIRST = R == 0, LAST = R == RI::NR - 1;
     constexpr bool ROWS = C == 0 && A == 0;  // a thread's elements are consecutive
     constexpr int CH = ROWS ? RR / 4 : 1;    // its 16-byte chunks
-    constexpr int XBITS = TT - RB;
-    constexpr BitMap M = make_map(OA, RB, !FIRST && !LAST);
+    constexpr int XBITS = T - RB;
+    constexpr BitMap M = make_map(T, OA, RB, !FIRST && !LAST);
     const FftLaunch &p = *geo.p;
     const uint32_t lo = (C == 0) ? 0u : LO ? (uint32_t)LO : p.lo;
     const uint32_t sh = lo + A;  // global bit of the round's first owned bit
@@ -480,8 +480,8 @@ __device__ __forceinline__ void roundT(uint32_t *sm, const GeoT &geo) {
                 const uint32_t *src;
                 uint32_t *dst;
                 const bool whole = G >= RB + 5 || geo.nc >= (uint32_t)(RB + 5);
-                const bool there = tile_column<G, C>(geo, region, src, dst);
-                src += (tile_index<G, C, LO>(geo, region) & p.src_mask) + 4u * lane;
+                const bool there = tile_column<G, C, T>(geo, region, src, dst);
+                src += (tile_index<G, C, LO, T>(geo, region) & p.src_mask) + 4u * lane;
 #pragma unroll
                 for (int i = 0; i < CH; i++) {
                     uint4 t = make_uint4(0, 0, 0, 0);
@@ -490,16 +490,16 @@ __device__ __forceinline__ void roundT(uint32_t *sm, const GeoT &geo) {
                     } else {
                         const uint32_t e = region + 4u * (i * 32u + lane);
                         const uint32_t *s2;
-                        if (tile_column<G, C>(geo, e, s2, dst))
-                            t = __ldg(reinterpret_cast<const uint4 *>(s2 + (tile_index<G, C, LO>(geo, e) & p.src_mask)));
+                        if (tile_column<G, C, T>(geo, e, s2, dst))
+                            t = __ldg(reinterpret_cast<const uint4 *>(s2 + (tile_index<G, C, LO, T>(geo, e) & p.src_mask)));
                     }
                     v[grp][4 * i] = t.x; v[grp][4 * i + 1] = t.y; v[grp][4 * i + 2] = t.z; v[grp][4 * i + 3] = t.w;
                 }
             } else {
                 const uint32_t *src;
                 uint32_t *dst;
-                const bool there = tile_column<G, C>(geo, jb, src, dst);
-                src += tile_index<G, C, LO>(geo, jb) & p.src_mask;
+                const bool there = tile_column<G, C, T>(geo, jb, src, dst);
+                src += tile_index<G, C, LO, T>(geo, jb) & p.src_mask;
 #pragma unroll
                 for (int m = 0; m < RR; m++) v[grp][m] = there ? __ldg(src + ((size_t)m << sh)) : 0u;
             }
@@ -507,7 +507,7 @@ __device__ __forceinline__ void roundT(uint32_t *sm, const GeoT &geo) {
     }
     auto group = [&](int grp, uint32_t (&w)[RR]) {
         const uint32_t jb = jt | deposit<XBITS>((uint32_t)grp << W, M);
-        const uint32_t gb = tile_index<G, C, LO>(geo, jb);
+        const uint32_t gb = tile_index<G, C, LO, T>(geo, jb);
         const uint32_t region = jb & ~((32u << RB) - 1u);
         const uint32_t sj = swz_c(jb);
         if constexpr (FIRST && ROWS) {
@@ -548,8 +548,8 @@ __device__ __forceinline__ void roundT(uint32_t *sm, const GeoT &geo) {
                         make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
                 __syncwarp();
                 const bool whole = G >= RB + 5 || geo.nc >= (uint32_t)(RB + 5);
-                const bool there = tile_column<G, C>(geo, region, src, dst);
-                dst += tile_index<G, C, LO>(geo, region) + 4u * lane;
+                const bool there = tile_column<G, C, T>(geo, region, src, dst);
+                dst += tile_index<G, C, LO, T>(geo, region) + 4u * lane;
 #pragma unroll
                 for (int i = 0; i < CH; i++) {
                     const uint32_t q = i * 32u + lane, e = region + 4u * q;
@@ -558,11 +558,11 @@ __device__ __forceinline__ void roundT(uint32_t *sm, const GeoT &geo) {
                         if (there) *reinterpret_cast<uint4 *>(dst + 128u * i) = t;
                     } else {
                         uint32_t *d2;
-                        if (tile_column<G, C>(geo, e, src, d2))
-                            *reinterpret_cast<uint4 *>(d2 + tile_index<G, C, LO>(geo, e)) = t;
+                        if (tile_column<G, C, T>(geo, e, src, d2))
+                            *reinterpret_cast<uint4 *>(d2 + tile_index<G, C, LO, T>(geo, e)) = t;
                     }
                 }
-            } else if (tile_column<G, C>(geo, jb, src, dst)) {
+            } else if (tile_column<G, C, T>(geo, jb, src, dst)) {
                 dst += gb;
 #pragma unroll
                 for (int m = 0; m < RR; m++) dst[(size_t)m << sh] = w[m];
@@ -578,11 +578,11 @@ __device__ __forceinline__ void roundT(uint32_t *sm, const GeoT &geo) {
     }
 }
 
-template <int G, int C, bool INV, int E, int LO, int... Rs>
+template <int G, int C, bool INV, int E, int LO, int T, int... Rs>
 __device__ __forceinline__ void roundsT(uint32_t *sm, const GeoT &geo, std::integer_sequence<int, Rs...>) {
     (
         [&] {
-            roundT<G, C, INV, Rs, E, LO>(sm, geo);
+            roundT<G, C, INV, Rs, E, LO, T>(sm, geo);
             if constexpr (Rs + 1 < RoundT<G, INV, 0, E>::NR) __syncthreads();
         }(),
         ...);
@@ -592,22 +592,22 @@ __device__ __forceinline__ void roundsT(uint32_t *sm, const GeoT &geo, std::inte
 // shared memory), measured 2292 vs 2231 columns/s at log 24 against two CTAs per SM
 // with 112-128 registers, and 2132 with four CTAs per SM (64 registers). 2^5 elements
 // a thread (512 threads): two CTAs per SM (64 registers; at three it spills).
-template <int G, int C, bool INV, int E, int LO>
-__global__ void __launch_bounds__(1 << (TT - E), E == 6 ? 3 : 2) fftT_kernel(const __grid_constant__ FftLaunch p, uint32_t n_cols) {
+template <int G, int C, bool INV, int E, int LO, int T>
+__global__ void __launch_bounds__(1 << (T - E), E == 6 ? 3 : 2) fftT_kernel(const __grid_constant__ FftLaunch p, uint32_t n_cols) {
     extern __shared__ __align__(16) uint32_t sm[];
     chain_wait();
     GeoT geo;
     geo.p = &p;
     geo.n_cols = n_cols;
-    geo.nc = min(p.N, (uint32_t)TT);
+    geo.nc = min(p.N, (uint32_t)T);
     if constexpr (C == 0) {
-        if (G == TT || p.N >= (uint32_t)TT) {
+        if (G == T || p.N >= (uint32_t)T) {
             // tile position major, column minor
-            const uint32_t T = blockIdx.x / n_cols;
-            geo.col = blockIdx.x - T * n_cols;
-            geo.gfix = T << TT;
+            const uint32_t at = blockIdx.x / n_cols;
+            geo.col = blockIdx.x - at * n_cols;
+            geo.gfix = at << T;
         } else {
-            geo.col = blockIdx.x << (TT - p.N);
+            geo.col = blockIdx.x << (T - p.N);
             geo.gfix = 0;
         }
     } else {
@@ -619,25 +619,25 @@ __global__ void __launch_bounds__(1 << (TT - E), E == 6 ? 3 : 2) fftT_kernel(con
     const FftColumn fc = fft_col(p, geo.col);
     geo.src = fc.src;
     geo.dst = fc.dst;
-    roundsT<G, C, INV, E, LO>(sm, geo, std::make_integer_sequence<int, RoundT<G, INV, 0, E>::NR>{});
+    roundsT<G, C, INV, E, LO, T>(sm, geo, std::make_integer_sequence<int, RoundT<G, INV, 0, E>::NR>{});
 }
 
-template <int G, int C, bool INV, int E, int LO>
+template <int G, int C, bool INV, int E, int LO, int T = TT>
 int launchT_e(const FftLaunch &p, uint32_t n_cols, cudaStream_t st) {
     constexpr int NR = RoundT<G, INV, 0, E>::NR;
-    const size_t smem = NR > 1 || C == 0 ? (sizeof(uint32_t) << TT) : 0;
-    auto kern = fftT_kernel<G, C, INV, E, LO>;
+    const size_t smem = NR > 1 || C == 0 ? (sizeof(uint32_t) << T) : 0;
+    auto kern = fftT_kernel<G, C, INV, E, LO, T>;
     static std::atomic<uint64_t> attr_set{0};
     int rc = once_per_device(attr_set, [&] {
         STWO_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)(sizeof(uint32_t) << TT)));
+                                           (int)(sizeof(uint32_t) << T)));
         return (int)STWO_OK;
     });
     if (rc) return rc;
-    const uint64_t blocks = p.N >= (uint32_t)TT ? (uint64_t)n_cols << (p.N - TT)
-                                                : ((uint64_t)n_cols + (1u << (TT - p.N)) - 1) >> (TT - p.N);
+    const uint64_t blocks = p.N >= (uint32_t)T ? (uint64_t)n_cols << (p.N - T)
+                                                : ((uint64_t)n_cols + (1u << (T - p.N)) - 1) >> (T - p.N);
     STWO_REQUIRE(blocks < (1ull << 31), STWO_ERR_UNSUPPORTED_SIZE, "fft launch of %llu tiles", (unsigned long long)blocks);
-    launch_chained(kern, (unsigned)blocks, 1 << (TT - E), smem, st, p, n_cols);
+    launch_chained(kern, (unsigned)blocks, 1 << (T - E), smem, st, p, n_cols);
     STWO_LAUNCH_CHECK("fftT_kernel");
     return STWO_OK;
 }
@@ -656,6 +656,21 @@ inline int fft_ept_log(bool contiguous, uint32_t N) {
 
 template <int G, int C, bool INV, int LO = 0>
 int launchT_t(const FftLaunch &p, uint32_t n_cols, cudaStream_t st) {
+    // Launches whose tiles all run at once take as long as one thread's work, so they spread it
+    // over more threads: transforms of 2^11..2^13 points as tiles of 2^12 elements with 16 a
+    // thread or of 2^13 with 32, up to two tiles an SM (B200, us, interpolate / evaluate at
+    // blowup 2: 64 x 2^12 14.9 / 15.7 -> 8.6 / 8.6, 1 x 2^13 15.0 / 16.4 -> 10.8 / 12.2, 128 x
+    // 2^13 15.9 / 17.1 -> 11.6 / 14.8; a 64 x 2^12 proof 536 -> 511), and passes of 14 layers
+    // 32 a thread, up to one tile an SM (1 x 2^14 15.5 / 16.9 -> 14.7 / 14.8, 32 x 2^16 21.5 /
+    // 29.7 -> 19.4 / 29.7; 16 a thread the same).
+    if constexpr (C == 0 && G >= 11 && G <= 13) {
+        constexpr int T = G == 13 ? 13 : 12;
+        if ((uint64_t)n_cols << p.N <= (2ull * device_sm_count()) << T)
+            return launchT_e<G, C, INV, T - 8, 0, T>(p, n_cols, st);
+    }
+    if constexpr (C == 0 && G == TT)
+        if ((uint64_t)n_cols << p.N <= (uint64_t)device_sm_count() << TT)
+            return launchT_e<G, C, INV, 5, 0>(p, n_cols, st);
     if constexpr (C > 0 || G >= 11)
         if (fft_ept_log(C == 0, p.N) == 5) return launchT_e<G, C, INV, 5, 0>(p, n_cols, st);
     return launchT_e<G, C, INV, 6, LO>(p, n_cols, st);
