@@ -214,10 +214,13 @@ __global__ void fs_comp_kernel(ProofState *s, const uint32_t *root, size_t js) {
 // values, then the composition's 4 coordinates) and draws the quotient coefficient;
 // then the quotient kernels' sample-dependent parameters of both column groups.
 // The sampled values are first staged in shared memory (up to OODS_STAGED of them), so
-// that the serial hash reads each chunk without an L2 round trip; the constraint check
-// runs on another warp while thread 0 hashes. vsh: vanishing_shift(L), from the host.
+// that the serial hash reads each chunk without an L2 round trip; the constraint sum and its
+// check run on the other warps while thread 0 hashes, and both groups' parameters are filled
+// in one go (the OODS evaluation and this step with 64, 128 and 256 columns: 49 -> 41,
+// 90 -> 72 and 369 -> 350 us). vsh: vanishing_shift(L), from the host.
 constexpr uint32_t OODS_STAGED = 1024;
-__global__ void __launch_bounds__(256) fs_oods_kernel(ProofState *s, const qm31 *sampled, const qm31 *powers,
+constexpr uint32_t OODS_THREADS = 256;
+__global__ void __launch_bounds__(OODS_THREADS) fs_oods_kernel(ProofState *s, const qm31 *sampled, const qm31 *powers,
                                                       uint32_t N, uint32_t L, cpoint vsh, QuotParamsDev *q_comp,
                                                       QuotParamsDev *q_trace, size_t js) {
     chain_wait();
@@ -236,19 +239,29 @@ __global__ void __launch_bounds__(256) fs_oods_kernel(ProofState *s, const qm31 
         for (uint32_t i = threadIdx.x; i < n_vals; i += blockDim.x) staged[i] = sampled[i];
     __syncthreads();
     const qm31 *vals = stage ? staged : sampled;
-    qm31 part = qm31_zero();
-    for (uint32_t i = threadIdx.x; i + 2 < N; i += blockDim.x) {
-        const qm31 cons = qm31_sub(qm31_add(qm31_mul(vals[i], vals[i]), qm31_mul(vals[i + 1], vals[i + 1])), vals[i + 2]);
-        part = qm31_add(part, qm31_mul(cons, powers[N - 3 - i]));
-    }
-    const qm31 acc = block_sum_qm31(part, sh);
     const qm31 ox = s->oods[0], oy = s->oods[1];
+    const uint32_t warp = threadIdx.x >> 5;
+    if (warp > 0) {
+        qm31 part = qm31_zero();
+        for (uint32_t i = threadIdx.x - 32; i + 2 < N; i += OODS_THREADS - 32) {
+            const qm31 cons =
+                qm31_sub(qm31_add(qm31_mul(vals[i], vals[i]), qm31_mul(vals[i + 1], vals[i + 1])), vals[i + 2]);
+            part = qm31_add(part, qm31_mul(cons, powers[N - 3 - i]));
+        }
+        part = warp_sum_qm31(part);
+        if ((threadIdx.x & 31u) == 0) sh[warp] = part;
+        asm volatile("bar.sync 1, %0;" ::"n"(OODS_THREADS - 32) : "memory");  // the warps but the first
+    }
     if (threadIdx.x == 0) {
-        fs::ch_mix_felts(s->ch, vals, n_vals);
-        const qm31 qrc = fs::ch_draw_felt(s->ch, s->error);
+        fs::DevChannel ch = s->ch;
+        fs::ch_mix_felts(ch, vals, n_vals);
+        const qm31 qrc = fs::ch_draw_felt(ch, s->error);
+        s->ch = ch;
         s->qrc = qrc;
         qrc_sh = qrc;
     } else if (threadIdx.x == 32) {
+        qm31 acc = sh[1];
+        for (uint32_t w = 2; w < OODS_THREADS / 32; w++) acc = qm31_add(acc, sh[w]);
         // composition value: from_partial_evals over the basis 1, i, u, iu
         const qm31 basis[4] = {{{1, 0}, {0, 0}}, {{0, 1}, {0, 0}}, {{0, 0}, {1, 0}}, {{0, 0}, {0, 1}}};
         qm31 comp = qm31_zero();
@@ -263,9 +276,7 @@ __global__ void __launch_bounds__(256) fs_oods_kernel(ProofState *s, const qm31 
     }
     __syncthreads();
     if (threadIdx.x == 0) s->error |= bad_sh;
-    const qm31 qrc = qrc_sh;
-    quot_fill_batch_block(*q_comp, 0, qrc, ox, oy, vals + N, 4, 0, sh);
-    quot_fill_batch_block(*q_trace, 0, qrc, ox, oy, vals, N, 0, sh);
+    quot_fill_two_block(*q_comp, vals + N, 4, *q_trace, vals, N, qrc_sh, ox, oy, sh);
 }
 
 // Channel step after an FRI tree: mix its root, draw the folding alpha.
@@ -1291,7 +1302,7 @@ int prove_jobs(const Job &j, uint32_t K, const uint32_t *const *a0_in, const uin
         // ---- 3. out-of-domain sampling
         PV_TRY(eval_at_points_dev_async(dev_at(off_eap), eap_n, eap_iter, eap_total, dstate->oods, dsampled,
                                         eap_partials, dtickets, K, js, st));
-        launch_chained(fs_oods_kernel, K, 256, 0, st, dstate, dsampled, powers, N, L, vanishing_shift(L), dqc, dqt, js);
+        launch_chained(fs_oods_kernel, K, OODS_THREADS, 0, st, dstate, dsampled, powers, N, L, vanishing_shift(L), dqc, dqt, js);
         STWO_LAUNCH_CHECK("fs_oods_kernel");
         PV_TRY(record(3, capturing));
 

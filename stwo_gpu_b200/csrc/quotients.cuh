@@ -95,52 +95,64 @@ __host__ __device__ inline void quot_scale_batches(QP &p, uint32_t n_batches) {
     }
 }
 
-// Sum of one QM31 per thread over a CTA of blockDim.x <= 1024 threads; every thread
-// gets the sum. sh: 32 QM31 of shared memory.
-__device__ inline qm31 block_sum_qm31(qm31 v, qm31 *sh) {
+// Sum of one QM31 per lane over the warp; every lane gets the sum.
+__device__ __forceinline__ qm31 warp_sum_qm31(qm31 v) {
+#pragma unroll
     for (int m = 16; m >= 1; m >>= 1) {
         v.a.a = m31_add(v.a.a, __shfl_xor_sync(0xffffffffu, v.a.a, m));
         v.a.b = m31_add(v.a.b, __shfl_xor_sync(0xffffffffu, v.a.b, m));
         v.b.a = m31_add(v.b.a, __shfl_xor_sync(0xffffffffu, v.b.a, m));
         v.b.b = m31_add(v.b.b, __shfl_xor_sync(0xffffffffu, v.b.b, m));
     }
-    __syncthreads();  // sh may hold a previous call's values
-    if ((threadIdx.x & 31u) == 0) sh[threadIdx.x >> 5] = v;
-    __syncthreads();
-    qm31 s = qm31_zero();
-    for (uint32_t w = 0; w < (blockDim.x + 31) / 32; w++) s = qm31_add(s, sh[w]);
-    return s;
+    return v;
 }
 
-// quot_fill_batch by a whole CTA: thread t takes samples t, t + T, ... with
-// alpha = rc^(j+1), and the a / b sums are reduced across the CTA. For the prover's
-// single-batch groups (no quot_scale_batches step is needed with one batch).
+// quot_fill_batch of two single-batch groups at one point by a CTA of 256 threads: thread t
+// takes samples t, t + 256, ... of both with alpha = rc^(j+1) (the first group has at most
+// 256), and the a / b sums of both are reduced across the CTA together. For the prover's
+// groups: no quot_scale_batches step is needed with one batch, nor the batch coefficient
+// it reads. sh: 32 QM31 of shared memory.
 template <class QP>
-__device__ inline void quot_fill_batch_block(QP &p, uint32_t b, qm31 rc, qm31 px, qm31 py, const qm31 *vals,
-                                             uint32_t count, uint32_t off, qm31 *sh) {
-    const uint32_t T = blockDim.x;
+__device__ inline void quot_fill_two_block(QP &p0, const qm31 *vals0, uint32_t count0, QP &p1, const qm31 *vals1,
+                                           uint32_t count1, qm31 rc, qm31 px, qm31 py, qm31 *sh) {
+    constexpr uint32_t T = 256;
+    const uint32_t tid = threadIdx.x;
     const qm31 c0 = qm31_sub(qm31_conj(py), py);
-    const qm31 step = qm31_pow(rc, T);
-    qm31 alpha = qm31_pow(rc, threadIdx.x + 1), as = qm31_zero(), bs = qm31_zero();
-    for (uint32_t j = threadIdx.x; j < count; j += T) {
-        const qm31 v = vals[j];
-        qm31 a = qm31_sub(qm31_conj(v), v);
-        qm31 bb = qm31_sub(qm31_mul(v, c0), qm31_mul(a, py));
-        a = qm31_mul(alpha, a);
-        bb = qm31_mul(alpha, bb);
-        const qm31 c = qm31_mul(alpha, c0);
-        as = qm31_add(as, a);
-        bs = qm31_add(bs, bb);
-        p.c2[off + j] = c;
-        alpha = qm31_mul(alpha, step);
+    qm31 alpha = qm31_pow(rc, tid + 1);
+    qm31 sum[4] = {qm31_zero(), qm31_zero(), qm31_zero(), qm31_zero()};  // a and b of group 0, of group 1
+    auto fill = [&](QP &p, const qm31 *vals, uint32_t j, qm31 c, qm31 &as, qm31 &bs) {
+        const qm31 v = vals[j], a = qm31_sub(qm31_conj(v), v);
+        as = qm31_add(as, qm31_mul(alpha, a));
+        bs = qm31_add(bs, qm31_mul(alpha, qm31_sub(qm31_mul(v, c0), qm31_mul(a, py))));
+        p.c2[j] = c;
+    };
+    if (tid < count0) fill(p0, vals0, tid, qm31_mul(alpha, c0), sum[0], sum[1]);
+    if (tid < count1) fill(p1, vals1, tid, qm31_mul(alpha, c0), sum[2], sum[3]);
+    if (count1 > T) {
+        const qm31 step = qm31_pow(rc, T);
+        for (uint32_t j = tid + T; j < count1; j += T) {
+            alpha = qm31_mul(alpha, step);
+            fill(p1, vals1, j, qm31_mul(alpha, c0), sum[2], sum[3]);
+        }
     }
-    as = block_sum_qm31(as, sh);
-    bs = block_sum_qm31(bs, sh);
-    if (threadIdx.x == 0) {
-        quot_fill_point(p, b, px, py);
-        p.batch_coeff[b] = qm31_pow(rc, count);
-        p.a_sum[b] = as;
-        p.b_sum[b] = bs;
+    __syncthreads();  // sh may hold earlier values
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const qm31 w = warp_sum_qm31(sum[q]);
+        if ((tid & 31u) == 0) sh[8 * q + (tid >> 5)] = w;
+    }
+    __syncthreads();
+    if (tid == 0 || tid == 32) {
+        QP &p = tid ? p1 : p0;
+        const qm31 *s = sh + (tid ? 16 : 0);
+        qm31 as = qm31_zero(), bs = qm31_zero();
+        for (int w = 0; w < 8; w++) {
+            as = qm31_add(as, s[w]);
+            bs = qm31_add(bs, s[8 + w]);
+        }
+        quot_fill_point(p, 0, px, py);
+        p.a_sum[0] = as;
+        p.b_sum[0] = bs;
     }
 }
 
