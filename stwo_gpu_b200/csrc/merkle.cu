@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(256) merkle_layer_kernel(uint32_t log_size, co
 // ceiling (81% of the slots) where it is dense, so both the instructions and the number of
 // copies count. Layers of four columns (the QM31 columns of the composition and of FRI,
 // half of their trees' compressions) take a form without the 120 additions of zero words;
-// full and padded chunks share one copy. B200, us: 4 columns at each of 2^12..2^22 643 ->
+// full and padded chunks share one copy (but see launch_tree). B200, us: 4 columns at each of 2^12..2^22 643 ->
 // 573, 4 x 2^22 427 -> 388, 4 x 2^20 145 -> 134, 101 x 2^18 (a padded chunk) 152 -> 137;
 // 64 x 2^22 897 -> 896. Further copies cost more than they save: a zero-state form for
 // leaves beside this one 412 at 4 x 2^22, an eight-word form 659 over the mixed tree; one
@@ -131,7 +131,8 @@ struct TreeParams {
 };
 
 
-template <int THREADS>
+// FEW: layers of fewer than 16 columns take their one padded chunk by a copy of its own.
+template <int THREADS, bool FEW>
 __device__ __forceinline__ void merkle_unit(const TreeParams &p, const TreeBand &bd, uint32_t u,
                                             uint4 (*thin)[THREADS][2], uint32_t one) {
     const uint32_t job = blockIdx.y;
@@ -179,6 +180,12 @@ __device__ __forceinline__ void merkle_unit(const TreeParams &p, const TreeBand 
 #pragma unroll
                 for (int w = 0; w < 4; w++) m4[w] = __ldg(ct[w] + i);
                 compress<blake::ADD_FMA, 4, false, true>(h, m4, one);
+            } else if (FEW && nc < 16) {
+                if (nc) {
+#pragma unroll
+                    for (uint32_t w = 0; w < 16; w++) m[w] = w < nc ? __ldg(ct[w] + i) : 0u;
+                    compress<blake::ADD_FMA, 16, false, true>(h, m, one);
+                }
             } else {
                 // one loop for full chunks and the zero-padded last one (see above)
 #pragma unroll 1
@@ -208,14 +215,14 @@ __device__ __forceinline__ void merkle_unit(const TreeParams &p, const TreeBand 
     }
 }
 
-template <int THREADS>
+template <int THREADS, bool FEW>
 __global__ void __launch_bounds__(THREADS) merkle_tree_kernel(const __grid_constant__ TreeParams p, uint32_t one) {
     __shared__ uint4 thin[2][THREADS][2];
     __shared__ uint32_t next;
     chain_wait();
     uint32_t b = 0, u = blockIdx.x;
     for (;;) {
-        merkle_unit<THREADS>(p, p.band[b], u, thin, one);
+        merkle_unit<THREADS, FEW>(p, p.band[b], u, thin, one);
         if (b + 1 >= p.n_bands) return;
         const TreeBand &up = p.band[b + 1];
         const uint32_t parent = u / up.fan;
@@ -287,8 +294,23 @@ int plan_tree_bands(uint32_t max_log, TreePlan &tp) {
 }
 
 template <int THREADS>
-void launch_tree(const TreeParams &p, uint32_t blocks, uint32_t jobs, cudaStream_t st) {
-    launch_chained(merkle_tree_kernel<THREADS>, dim3(blocks, jobs), THREADS, 0, st, p, 1u);
+void launch_tree(const TreeParams &p, uint32_t max_log, uint32_t blocks, uint32_t jobs, cudaStream_t st) {
+    // FEW: small trees of several sizes whose layers all have fewer than 16 columns, not only
+    // four. 1, 13 columns at each of 2^12..2^16 take 42.0, 43.8 us with the shared copy and
+    // 40.4, 41.6 with FEW (one copy of each kind of chunk: 40.8, 42.6), 1, 13 at each of
+    // 2^8..2^12 35.6, 37.4 and 32.4, 33.3. Not for leaves alone (13 x 2^14 26.6 and 27.3), nor
+    // with 16 columns (2^12..2^16: 41.6 and 42.7); from 2^17 leaves the dense layers decide
+    // (13 at each of 2^16..2^20 188.7 and 194.2). The gain is where the code lies, not its
+    // length: a kernel with the padded copy and no loop is no faster than the shared copy.
+    bool few = max_log <= 16;
+    int inner = 0;  // layers with children and a chunk
+    for (uint32_t l = 0; l <= max_log; l++) {
+        few = few && p.n_cols[l] < 16;
+        inner += l < max_log && p.n_cols[l] != 0 && p.n_cols[l] != 4;
+    }
+    few = few && inner >= 2;
+    launch_chained(few ? merkle_tree_kernel<THREADS, true> : merkle_tree_kernel<THREADS, false>, dim3(blocks, jobs), THREADS,
+                   0, st, p, 1u);
 }
 
 template <int CAP>
@@ -334,9 +356,9 @@ int merkle_tree_dev_async(uint32_t max_log, const uint32_t *const *const *level_
     STWO_REQUIRE(jobs >= 1 && jobs <= 65535, STWO_ERR_INVALID_ARGUMENT, "merkle trees per launch: %u", jobs);
     p.js = js;
     auto launch = [&](uint32_t blocks) {
-        if (tp.threads == 512) launch_tree<512>(p, blocks, jobs, st);
-        else if (tp.threads == 128) launch_tree<128>(p, blocks, jobs, st);
-        else launch_tree<256>(p, blocks, jobs, st);
+        if (tp.threads == 512) launch_tree<512>(p, max_log, blocks, jobs, st);
+        else if (tp.threads == 128) launch_tree<128>(p, max_log, blocks, jobs, st);
+        else launch_tree<256>(p, max_log, blocks, jobs, st);
     };
     if (tickets && n_tickets >= tp.n_tickets) {
         for (uint32_t b = 0; b < tp.n_bands; b++) p.band[b] = tp.band[b];

@@ -23,3 +23,22 @@ def test_tree_layers_match_oracle(stwo, oracle, nc):
     want = oracle.merkle_commit(cols)
     for l in range(12):
         assert (layers[l].to_numpy().reshape(-1, 8) == want[l]).all(), l
+
+
+@pytest.mark.parametrize("per", [(15, 1, 1, 1), (15, 16, 1, 1), (4, 3, 0, 2), (1, 4, 4, 5)])
+@pytest.mark.parametrize("top", [2, 16, 17])
+def test_small_trees_of_several_sizes_match_oracle(stwo, oracle, top, per):
+    """Both sides of the rule for small trees: 16 and 17 as the largest log size, 15 and 16
+    columns, one and two inner layers with other than four."""
+    L = stwo._lib
+    r = rng(3200 + top)
+    logs = [lg for n, lg in zip(per, (top, top - 1, top // 2, 0)) for _ in range(n)]
+    cols = [m31(r, 1 << lg) for lg in logs]
+    bufs = [stwo.BaseFieldVec.from_numpy(c) for c in cols]
+    layers = [stwo.BaseFieldVec.new_uninitialized(8 << l) for l in range(top + 1)]
+    L.check(L.lib().stwo_merkle_commit_tree(L.ptr_array([b.device_ptr for b in bufs]), L.u32_array(logs), len(logs),
+                                            top, L.ptr_array([x.device_ptr for x in layers]), None))
+    L.check(L.lib().stwo_stream_synchronize(None))
+    want = oracle.merkle_commit(cols)
+    for l in range(top + 1):
+        assert (layers[l].to_numpy().reshape(-1, 8) == want[l]).all(), l
