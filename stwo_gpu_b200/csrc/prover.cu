@@ -331,7 +331,7 @@ __device__ void fs_last(ProofState *s, const uint32_t *const c[4], uint32_t log)
 // through distributed shared memory and finishes; alpha goes back the same way. A CTA's folded
 // values are its own eighth of the next layer. Smaller layers are CTA 0's alone. (One CTA of
 // 1024 threads hashed the 1024 leaves of log size 10 in 12.8k cycles, and log sizes 11 to 13
-// took three launches a layer: a 64-column x 2^12 proof FIGURES.)
+// took three launches a layer: the FRI phase of a 64-column x 2^12 proof 254 -> 240 us.)
 // Values this kernel wrote are read back with plain (coherent) loads after a
 // barrier; nothing is read through the non-coherent path except the trace quotient
 // and the twiddles.
