@@ -891,9 +891,7 @@ uint64_t job_device_bytes(const Job &j, bool own_twiddles) {
     auto tickets = [&](uint32_t log) { return r(4 * std::max<uint64_t>(merkle_tree_tickets(log), 1)); };
     b += tickets(j.L + j.B) + 2 * tickets(j.L + 1 + j.B);  // Merkle tree tickets
     for (uint32_t l = j.B; l <= j.L + j.B; l++) b += tickets(l);
-    const uint64_t words = (uint64_t)j.n_queries * ((j.L + 2 + j.B) * 8 * 3 * 8 + 2 * (j.N + 16));
-    b += r(words * sizeof(GatherReq)) + r(words * 4);     // decommitment gather
-    return b;
+    return b;  // (the decommitment gather's requests and words are pinned host memory)
 }
 
 // Timing events of one thread's proofs (reused; created on first use per device).
