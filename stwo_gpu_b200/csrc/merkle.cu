@@ -295,20 +295,30 @@ int plan_tree_bands(uint32_t max_log, TreePlan &tp) {
 
 template <int THREADS>
 void launch_tree(const TreeParams &p, uint32_t max_log, uint32_t blocks, uint32_t jobs, cudaStream_t st) {
-    // FEW: small trees of several sizes whose layers all have fewer than 16 columns, not only
-    // four. 1, 13 columns at each of 2^12..2^16 take 42.0, 43.8 us with the shared copy and
-    // 40.4, 41.6 with FEW (one copy of each kind of chunk: 40.8, 42.6), 1, 13 at each of
-    // 2^8..2^12 35.6, 37.4 and 32.4, 33.3. Not for leaves alone (13 x 2^14 26.6 and 27.3), nor
-    // with 16 columns (2^12..2^16: 41.6 and 42.7); from 2^17 leaves the dense layers decide
-    // (13 at each of 2^16..2^20 188.7 and 194.2). The gain is where the code lies, not its
-    // length: a kernel with the padded copy and no loop is no faster than the shared copy.
-    bool few = max_log <= 16;
+    // FEW: trees of up to 2^19 leaves and of several sizes whose layers all have fewer than 16
+    // columns, not only four; the larger the tree, the more such inner layers it takes, since
+    // its dense layers run better with the shared copy. B200, us, the call alone and hot,
+    // shared copy and FEW, 1 / 3 / 13 columns at each size:
+    //   2^8..2^13               40.2 / 41.1 / 42.5 and 36.4 / 38.1 / 37.8
+    //   2^4..2^16               68.4 / 67.3 / 72.1 and 59.0 / 60.6 / 62.3
+    //   2^14..2^16 (left out)   36.1 / 35.9 / 36.6 and 36.2 / 36.6 / 37.8
+    //   2^4..2^17               79.6 / 82.0 / 84.8 and 72.2 / 72.6 / 74.0
+    //   2^13..2^17              53.8 / 54.2 / 53.3 and 52.4 / 52.3 / 52.7
+    //   2^14..2^17 (left out)   51.3 / 51.1 / 51.2 and 50.4 / 51.1 / 51.7
+    //   2^4..2^18               122.0 / 122.4 / 126.1 and 111.0 / 111.7 / 112.9
+    //   2^4..2^19               156.3 / 157.7 / 164.4 and 146.8 / 149.7 / 159.6
+    //   2^15..2^19 (left out)   115.0 / 114.4 / 118.8 and 114.7 / 115.4 / 120.7
+    //   2^12..2^20 (left out)   195.9 / 200.4 / 209.9 and 197.9 / 205.1 / 214.3
+    // Nor for leaves alone (13 x 2^14 26.6 and 27.3) or with 16 columns (2^12..2^16: 41.6 and
+    // 42.7). The gain is where the code lies, not its length: a kernel with the padded copy
+    // and no loop is no faster than the shared copy.
+    bool few = max_log <= 19;
     int inner = 0;  // layers with children and a chunk
     for (uint32_t l = 0; l <= max_log; l++) {
         few = few && p.n_cols[l] < 16;
         inner += l < max_log && p.n_cols[l] != 0 && p.n_cols[l] != 4;
     }
-    few = few && inner >= 2;
+    few = few && inner >= std::max(1, (int)max_log - 13);
     launch_chained(few ? merkle_tree_kernel<THREADS, true> : merkle_tree_kernel<THREADS, false>, dim3(blocks, jobs), THREADS,
                    0, st, p, 1u);
 }

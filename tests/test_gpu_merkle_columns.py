@@ -42,3 +42,23 @@ def test_small_trees_of_several_sizes_match_oracle(stwo, oracle, top, per):
     want = oracle.merkle_commit(cols)
     for l in range(top + 1):
         assert (layers[l].to_numpy().reshape(-1, 8) == want[l]).all(), l
+
+
+@pytest.mark.parametrize("top,inner", [(4, 1), (14, 1), (15, 1), (15, 2), (16, 2), (16, 3), (17, 3), (17, 4), (18, 4),
+                                       (18, 5), (19, 5), (19, 6), (20, 7)])
+def test_trees_of_many_sizes_match_oracle(stwo, oracle, top, inner):
+    """The rule's line over the tree's size: the inner layers it asks for up to 2^14 leaves, at
+    2^15..2^19, and none above. Columns of the given number of inner sizes, the first of them
+    with three, and four at one size more, whose layer the rule does not count."""
+    L = stwo._lib
+    r = rng(3300 + 10 * top + inner)
+    logs = [top, top] + [top - 1] * 3 + [top - 1 - k for k in range(1, inner)] + [top - 1 - inner] * 4
+    cols = [m31(r, 1 << lg) for lg in logs]
+    bufs = [stwo.BaseFieldVec.from_numpy(c) for c in cols]
+    layers = [stwo.BaseFieldVec.new_uninitialized(8 << l) for l in range(top + 1)]
+    L.check(L.lib().stwo_merkle_commit_tree(L.ptr_array([b.device_ptr for b in bufs]), L.u32_array(logs), len(logs),
+                                            top, L.ptr_array([x.device_ptr for x in layers]), None))
+    L.check(L.lib().stwo_stream_synchronize(None))
+    want = oracle.merkle_commit(cols)
+    for l in range(top + 1):
+        assert (layers[l].to_numpy().reshape(-1, 8) == want[l]).all(), l
