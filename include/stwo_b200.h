@@ -189,11 +189,13 @@ int stwo_precompute_twiddles(uint32_t root_initial_index, uint32_t root_step_siz
 /* In-place circle FFTs over columns of mixed sizes; column i has 2^log_sizes[i]
  * elements and its domain's half coset is a doubling of the tree's root coset.
  * Inverse FFTs include the 2^-log rescale.
- * Up to 64 columns travel in the launch parameters, and so does any number of columns
- * of one size at equal distances (the rows of a matrix). Beyond that, these three
- * calls copy the column table into a pool buffer with a stream-ordered copy from
- * pageable host memory. Such a call may not be recorded into a CUDA graph; the
- * prover's own calls pass a prebuilt device table and stay graph-capturable. */
+ * Up to 64 columns of a size travel in the launch parameters, and so does any number of
+ * them at equal distances, ascending and less than 16 GiB apart (the rows of a matrix in
+ * their order). Other sets of more than 64 columns of a size have their table copied into
+ * a pool buffer, stream-ordered, from host memory of the call's own: such a call returns
+ * STWO_ERR_INVALID_ARGUMENT on a stream that is being captured into a CUDA graph. The
+ * others may be captured (from 8 points on; a 2- or 4-point transform reads a twiddle back to the
+ * host). The prover's own calls pass a prebuilt device table. */
 int stwo_interpolate_columns(uint32_t *const *columns, const uint32_t *log_sizes, uint32_t n_columns,
                              const uint32_t *itwiddles, uint64_t tree_size, void *stream);
 int stwo_evaluate_columns(uint32_t *const *columns, const uint32_t *log_sizes, uint32_t n_columns,
@@ -257,8 +259,9 @@ int stwo_merkle_commit_layer(uint32_t log_size, const uint32_t *prev_layer, cons
  * sizes (at most max_log); a layer's columns are hashed in their order in `columns`.
  * layers: host array of max_log + 1 device buffers, layers[l] receiving the 2^l nodes
  * of layer l (16-byte aligned); layers[0] is the root. The column tables and the
- * kernel's tickets are staged through the library's pool with a copy from pageable
- * memory, so the call may not be recorded into a CUDA graph. */
+ * kernel's tickets are staged through the library's pool with a copy from host memory of
+ * the call's own, so the call returns STWO_ERR_INVALID_ARGUMENT on a stream that is being
+ * captured into a CUDA graph. */
 int stwo_merkle_commit_tree(const uint32_t *const *columns, const uint32_t *log_sizes, uint32_t n_columns,
                             uint32_t max_log, uint32_t *const *layers, void *stream);
 

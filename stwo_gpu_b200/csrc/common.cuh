@@ -133,6 +133,11 @@ cudaEvent_t last_wait_event();
 // buffer across threads. Valid until the thread's next host_stage call.
 int host_stage(size_t bytes, void **out);
 
+// An error while `st` is being captured, for calls that copy a table from memory of their
+// own: the copy would be recorded without complaint, and a replay would read that memory
+// long after the call has freed it.
+int refuse_capture(cudaStream_t st, const char *what);
+
 // Launch parameters that stwo_autotune measures and stwo_set_tunable sets
 // (process-wide; every value of a tunable computes the same results).
 enum Tunable {

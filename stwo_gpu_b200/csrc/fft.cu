@@ -963,6 +963,8 @@ int fft_columns_tab(const uint32_t *const *srcs, uint32_t *const *dsts, uint32_t
         } else if (dev_table) {
             table = static_cast<const FftColumn *>(dev_table);
         } else {
+            int crc = refuse_capture(st, "a transform of more than 64 columns not at equal distances");
+            if (crc) return crc;
             std::vector<FftColumn> h(n_cols);
             for (uint32_t i = 0; i < n_cols; i++) h[i] = FftColumn{srcs[i], dsts[i]};
             int arc = pool_alloc(&staged, sizeof(FftColumn) * n_cols, st);

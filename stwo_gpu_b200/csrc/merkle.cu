@@ -421,6 +421,8 @@ int stwo_merkle_commit_tree(const uint32_t *const *columns, const uint32_t *log_
     STWO_REQUIRE(max_log <= 30 && layers && (n_columns == 0 || (columns && log_sizes)), STWO_ERR_INVALID_ARGUMENT,
                  "merkle tree arguments");
     cudaStream_t st = as_stream(stream);
+    int crc = refuse_capture(st, "a whole Merkle tree");
+    if (crc) return crc;
     // Per-layer column tables, in one staged device buffer: layer l's columns in the
     // caller's order.
     std::vector<const uint32_t *> flat;

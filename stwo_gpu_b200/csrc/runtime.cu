@@ -85,6 +85,14 @@ int host_stage(size_t bytes, void **out) {
     return STWO_OK;
 }
 
+int refuse_capture(cudaStream_t st, const char *what) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    STWO_CUDA_TRY(cudaStreamIsCapturing(st, &status));
+    STWO_REQUIRE(status == cudaStreamCaptureStatusNone, STWO_ERR_INVALID_ARGUMENT,
+                 "%s may not be recorded into a CUDA graph: it stages a table from host memory", what);
+    return STWO_OK;
+}
+
 thread_local bool t_blocking_wait = false;
 thread_local uint32_t t_spin_us = 0;
 
