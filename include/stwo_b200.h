@@ -161,7 +161,8 @@ int stwo_reserve_device_memory(uint64_t bytes);
  * it is not NULL. Takes well under a second. */
 int stwo_autotune(char *report, size_t report_cap);
 /* Sets one tunable by name: fft_ept_contig_small / fft_ept_contig_large /
- * fft_ept_strided (5 or 6), merkle_sub_threads (128, 256 or 512), merkle_sub_spread
+ * fft_ept_strided (5 or 6; for launches of more tiles than the SMs take at once, smaller
+ * ones choose by themselves), merkle_sub_threads (128, 256 or 512), merkle_sub_spread
  * (0..5: log2 of the bottom-level nodes each thread hashes), eval_at_point_groups_log
  * (2..4: log2 of the 8192-coefficient groups each eval_at_point CTA folds; 0, the
  * default, chooses per launch), quotients_tensor_cores (0, 1 = the default, 2) and

@@ -642,15 +642,23 @@ int launchT_e(const FftLaunch &p, uint32_t n_cols, cudaStream_t st) {
     return STWO_OK;
 }
 
-// Elements per thread, 2^6 (256 threads per CTA) or 2^5 (512 threads): a tunable per
-// pass kind and domain size (stwo_autotune); 2^6 by default, measured faster at log 24
-// (2222 vs 2125 columns/s). STWO_FFT_EPT_LOG=5 sets every pass kind to 2^5.
-inline int fft_ept_log(bool contiguous, uint32_t N) {
+// Elements per thread in strided passes and contiguous ones of 11 layers and more, 2^6 (256
+// threads per CTA) or 2^5 (512 threads): a tunable per pass kind and domain size
+// (stwo_autotune); 2^6 by default, measured faster at log 24 (2222 vs 2125 columns/s). The
+// tunables govern launches of more tiles than launchT_t spreads over more threads;
+// STWO_FFT_EPT_LOG (5 or 6) sets one value for all of them, the small ones too. Contiguous
+// passes of 4..10 layers always take 2^6, generic ones (launch_pass) neither.
+inline int fft_ept_forced() {
     static const int forced = [] {
         const char *e = getenv("STWO_FFT_EPT_LOG");
-        return e ? atoi(e) : 0;
+        const int v = e ? atoi(e) : 0;
+        return v == 5 || v == 6 ? v : 0;
     }();
-    if (forced == 5 || forced == 6) return forced;
+    return forced;
+}
+
+inline int fft_ept_log(bool contiguous, uint32_t N) {
+    if (fft_ept_forced()) return fft_ept_forced();
     return tunable(!contiguous ? TUNE_FFT_EPT_STRIDED : N <= 20 ? TUNE_FFT_EPT_CONTIG_SMALL : TUNE_FFT_EPT_CONTIG_LARGE);
 }
 
@@ -665,11 +673,11 @@ int launchT_t(const FftLaunch &p, uint32_t n_cols, cudaStream_t st) {
     // 29.7 -> 19.4 / 29.7; 16 a thread the same).
     if constexpr (C == 0 && G >= 11 && G <= 13) {
         constexpr int T = G == 13 ? 13 : 12;
-        if ((uint64_t)n_cols << p.N <= (2ull * device_sm_count()) << T)
+        if (!fft_ept_forced() && (uint64_t)n_cols << p.N <= (2ull * device_sm_count()) << T)
             return launchT_e<G, C, INV, T - 8, 0, T>(p, n_cols, st);
     }
     if constexpr (C == 0 && G == TT)
-        if ((uint64_t)n_cols << p.N <= (uint64_t)device_sm_count() << TT)
+        if (!fft_ept_forced() && (uint64_t)n_cols << p.N <= (uint64_t)device_sm_count() << TT)
             return launchT_e<G, C, INV, 5, 0>(p, n_cols, st);
     if constexpr (C > 0 || G >= 11)
         if (fft_ept_log(C == 0, p.N) == 5) return launchT_e<G, C, INV, 5, 0>(p, n_cols, st);
