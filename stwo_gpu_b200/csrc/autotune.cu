@@ -2,8 +2,9 @@
 // device and keeps the fastest per size class (the Tunable table in common.cuh):
 //
 //   FFT elements per thread (2^5 or 2^6), separately for contiguous passes on domains
-//   up to 2^20, contiguous passes on larger domains, and strided passes; measured on 8
-//   columns interpolated at 2^18 / 2^22 and evaluated at blowup 4;
+//   up to 2^20, contiguous passes on larger domains, and strided passes; measured on 32
+//   columns of 2^18 or 8 of 2^22, interpolated and evaluated at blowup 4 (every one of
+//   these launches has more tiles than a launch that chooses for itself);
 //   Merkle layers per launch (CTA of 128, 256 or 512 threads); measured on a tree of
 //   64 columns x 2^19 leaves;
 //   Merkle bottom-level nodes per thread (2^1 .. 2^5); measured on a tree of 4
@@ -147,18 +148,18 @@ int stwo_autotune(char *report, size_t report_cap) {
     int rc = STWO_OK;
     {
         Buffers buf(st);
-        // ---- FFT: 8 columns, interpolate at 2^L, evaluate at 2^(L+2)
+        // ---- FFT: n columns, interpolate at 2^L, evaluate at 2^(L+2)
         const uint32_t NCOL = 8;
         struct Case {
-            uint32_t L;
+            uint32_t n, L;
             Tunable t;
             const char *name;
             int candidates[3];
         };
-        const Case cases[] = {{18, TUNE_FFT_EPT_CONTIG_SMALL, "fft_ept_contig_small", {6, 5, 0}},
-                              {22, TUNE_FFT_EPT_CONTIG_LARGE, "fft_ept_contig_large", {6, 5, 0}},
-                              {22, TUNE_FFT_EPT_STRIDED, "fft_ept_strided", {6, 5, 0}},
-                              {22, TUNE_FFT_MAX_STRIDED, "fft_max_strided_layers", {10, 7, 5}}};
+        const Case cases[] = {{32, 18, TUNE_FFT_EPT_CONTIG_SMALL, "fft_ept_contig_small", {6, 5, 0}},
+                              {NCOL, 22, TUNE_FFT_EPT_CONTIG_LARGE, "fft_ept_contig_large", {6, 5, 0}},
+                              {NCOL, 22, TUNE_FFT_EPT_STRIDED, "fft_ept_strided", {6, 5, 0}},
+                              {NCOL, 22, TUNE_FFT_MAX_STRIDED, "fft_max_strided_layers", {10, 7, 5}}};
         const uint32_t Dmax = 24;
         const uint64_t tsz = 1ull << (Dmax - 1);
         uint32_t *tw = buf.get(tsz), *itw = buf.get(tsz);
@@ -174,6 +175,12 @@ int stwo_autotune(char *report, size_t report_cap) {
         }
         for (const Case &cs : cases) {
             if (rc) break;
+            // the case's columns, from the front of the buffers on
+            std::vector<uint32_t *> cin(cs.n), cout(cs.n);
+            for (uint32_t c = 0; c < cs.n; c++) {
+                cin[c] = in[c % NCOL] + ((size_t)(c / NCOL) << cs.L);
+                cout[c] = out[c % NCOL] + ((size_t)(c / NCOL) << (cs.L + 2));
+            }
             float best_ms = 1e30f;
             int best = tunable(cs.t);
             char part[128];
@@ -183,10 +190,9 @@ int stwo_autotune(char *report, size_t report_cap) {
                 set_tunable(cs.t, v);
                 float ms = 0;
                 rc = time_best(st, [&] {
-                    int r = fft_columns(in.data(), in.data(), NCOL, cs.L, cs.L, itw, tsz, true, st);
+                    int r = fft_columns(cin.data(), cin.data(), cs.n, cs.L, cs.L, itw, tsz, true, st);
                     if (r) return r;
-                    std::vector<const uint32_t *> src(in.begin(), in.end());
-                    return fft_columns(src.data(), out.data(), NCOL, cs.L + 2, cs.L, tw, tsz, false, st);
+                    return fft_columns(cin.data(), cout.data(), cs.n, cs.L + 2, cs.L, tw, tsz, false, st);
                 }, &ms);
                 if (rc) break;
                 snprintf(part, sizeof(part), "%s\"%d\": %.4f", times.empty() ? "" : ", ", v, ms);

@@ -80,3 +80,14 @@ def test_forced_elements_per_thread_reach_every_pass():
         got = run(shapes, env={"STWO_FFT_EPT_LOG": str(value)})
         assert {(ept, t) for *_, ept, _, t, _ in got["passes"]} == {(value, 14)}
         assert got["digest"] == base["digest"]
+
+
+def test_autotune_times_both_candidates_of_every_launch():
+    """Every contiguous 14-layer launch shape that autotune times runs with 2^5 and with 2^6
+    elements a thread; one that the library chooses by itself would run with the same twice."""
+    got = run([[300, 4, 1]], autotune=True)
+    shapes = {}
+    for g, c, inv, ept, _, _, grid in got["passes"]:
+        if g == 14 and c == 0:
+            shapes.setdefault((inv, grid), set()).add(ept)
+    assert len(shapes) >= 4 and all(v == {5, 6} for v in shapes.values()), shapes
