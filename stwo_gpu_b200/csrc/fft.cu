@@ -644,8 +644,9 @@ int launchT_e(const FftLaunch &p, uint32_t n_cols, cudaStream_t st) {
 
 // Elements per thread in strided passes and contiguous ones of 11 layers and more, 2^6 (256
 // threads per CTA) or 2^5 (512 threads): a tunable per pass kind and domain size
-// (stwo_autotune); 2^6 by default, measured faster at log 24 (2222 vs 2125 columns/s). The
-// tunables govern launches of more tiles than launchT_t spreads over more threads;
+// (stwo_autotune); 2^6 by default, measured faster at most sizes (us, strided passes with 2^6
+// and 2^5, both compiled for their row distance: interpolate 64 x 2^20 281 and 302, 8 x 2^22
+// 156 and 161, 8 x 2^24 672 and 693; evaluate 8 x 2^24 637 and 622). The tunables govern launches of more tiles than launchT_t spreads over more threads;
 // STWO_FFT_EPT_LOG (5 or 6) sets one value for all of them, the small ones too. Contiguous
 // passes of 4..10 layers always take 2^6, generic ones (launch_pass) neither.
 inline int fft_ept_forced() {
@@ -680,7 +681,7 @@ int launchT_t(const FftLaunch &p, uint32_t n_cols, cudaStream_t st) {
         if (!fft_ept_forced() && (uint64_t)n_cols << p.N <= (uint64_t)device_sm_count() << TT)
             return launchT_e<G, C, INV, 5, 0>(p, n_cols, st);
     if constexpr (C > 0 || G >= 11)
-        if (fft_ept_log(C == 0, p.N) == 5) return launchT_e<G, C, INV, 5, 0>(p, n_cols, st);
+        if (fft_ept_log(C == 0, p.N) == 5) return launchT_e<G, C, INV, 5, LO>(p, n_cols, st);
     return launchT_e<G, C, INV, 6, LO>(p, n_cols, st);
 }
 

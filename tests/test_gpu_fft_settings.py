@@ -91,3 +91,16 @@ def test_autotune_times_both_candidates_of_every_launch():
         if g == 14 and c == 0:
             shapes.setdefault((inv, grid), set()).add(ept)
     assert len(shapes) >= 4 and all(v == {5, 6} for v in shapes.values()), shapes
+
+
+def test_strided_passes_of_both_settings_are_compiled_for_their_row_distance():
+    """The strided pass right above the bottom one (lowest layer 14, 6 layers and more), with 32
+    as with 64 elements a thread, so that the setting compares like with like."""
+    shapes = [[2, 20, 1], [1, 22, 1], [1, 23, 1]]
+    found = []
+    for value in (6, 5):
+        got = run(shapes, tunables=[["fft_ept_strided", value]])
+        strided = sorted({(g, c, inv, lowest, ept) for g, c, inv, ept, lowest, _, _ in got["passes"] if c})
+        assert strided and all(lowest == 14 and ept == value for *_, lowest, ept in strided), strided
+        found.append(([s[:3] for s in strided], got["digest"]))
+    assert found[0] == found[1]
