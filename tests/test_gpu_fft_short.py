@@ -69,3 +69,60 @@ def test_short_columns_match_oracle(stwo, oracle, log_size, ncols, blowup, gap, 
     L.check(lib.stwo_evaluate_columns(src, logs, ncols, tree.twiddles.device_ptr, len(tree.twiddles), None))
     L.check(lib.stwo_stream_synchronize(None))
     assert (buf.to_numpy().reshape(ncols + 1, n + gap)[:ncols, :n] == vals).all()
+
+
+def _check(stwo, oracle, log_size, ncols, blowup, seed):
+    """Interpolate and extend a matrix's rows with guard words behind and between them; rows at
+    both ends and at tile boundaries against the oracle, the others by the round trip."""
+    L = stwo._lib
+    lib = L.lib()
+    r = rng(seed)
+    n, m, gap = 1 << log_size, 1 << (log_size + blowup), 4
+    tree = stwo.CudaBackend.precompute_twiddles(stwo.CanonicCoset(log_size + blowup).half_coset())
+    tw, itw = tree.twiddles.to_numpy(), tree.itwiddles.to_numpy()
+    vals = m31(r, ncols * n).reshape(ncols, n)
+    _, buf = _matrix(stwo, vals, n + gap)
+    _, out = _matrix(stwo, np.full((ncols, m), GUARD, np.uint32), m + gap)
+    src = L.ptr_array([buf.device_ptr + 4 * (n + gap) * k for k in range(ncols)])
+    dst = L.ptr_array([out.device_ptr + 4 * (m + gap) * k for k in range(ncols)])
+    logs = L.u32_array([log_size] * ncols)
+    L.check(lib.stwo_interpolate_columns(src, logs, ncols, tree.itwiddles.device_ptr, len(tree.itwiddles), None))
+    L.check(lib.stwo_extend_evaluate_columns(src, logs, dst, blowup, ncols, tree.twiddles.device_ptr,
+                                             len(tree.twiddles), None))
+    L.check(lib.stwo_stream_synchronize(None))
+    got, ext = buf.to_numpy().reshape(ncols + 1, n + gap), out.to_numpy().reshape(ncols + 1, m + gap)
+    assert (got[ncols] == GUARD).all() and (ext[ncols] == GUARD).all()
+    assert (got[:, n:] == GUARD).all() and (ext[:, m:] == GUARD).all()
+
+    def oc(log):
+        c = stwo.CanonicCoset(log).half_coset()
+        return oracle.coset(c.initial_index, c.step_size, c.log_size)
+    per_tile = max(1, 1 << (14 - log_size))
+    for k in sorted({0, 1, per_tile - 1, per_tile, ncols // 2, ncols - 1} & set(range(ncols))):
+        coeffs = oracle.interpolate(oc(log_size), vals[k], itw)
+        assert (got[k, :n] == coeffs).all(), k
+        assert (ext[k, :m] == oracle.evaluate(oc(log_size + blowup), coeffs, tw)).all(), k
+    L.check(lib.stwo_evaluate_columns(src, logs, ncols, tree.twiddles.device_ptr, len(tree.twiddles), None))
+    L.check(lib.stwo_stream_synchronize(None))
+    assert (buf.to_numpy().reshape(ncols + 1, n + gap)[:ncols, :n] == vals).all()
+
+
+@pytest.mark.parametrize("log_size,ncols,blowup", [(11, 593, 1), (12, 297, 1), (13, 299, 1), (13, 297, 2)])
+def test_partial_last_tile_with_32_elements_a_thread(stwo, oracle, log_size, ncols, blowup):
+    """A 2^14 tile over 8, 4 or 2 columns by 512 threads, its last tile not full."""
+    L = stwo._lib
+    try:
+        L.check(L.lib().stwo_set_tunable(b"fft_ept_contig_small", 5))
+        _check(stwo, oracle, log_size, ncols, blowup, 7200 + log_size)
+    finally:
+        L.check(L.lib().stwo_set_tunable(b"fft_ept_contig_small", 6))
+
+
+@pytest.mark.parametrize("log_size,ncols,blowup", [
+    (4, 66, 10), (4, 70, 11), (5, 65, 9), (7, 67, 8), (8, 33, 7),
+    (10, 64, 4), (10, 65, 5), (10, 70, 4), (9, 3, 12),
+])
+def test_short_columns_extended_beyond_a_tile(stwo, oracle, log_size, ncols, blowup):
+    """Few coefficients evaluated on 2^14 points and more: the pass has 4..10 layers, its tile
+    lies within one column, and reads of the coefficients wrap within the tile."""
+    _check(stwo, oracle, log_size, ncols, blowup, 7300 + 20 * log_size + ncols)
