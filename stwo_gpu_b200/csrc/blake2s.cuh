@@ -45,10 +45,13 @@ __device__ __forceinline__ uint32_t add_on_fma(uint32_t c, uint32_t d, uint32_t 
 // Where the additions of G go:
 //  * ADD_FMA: all on the FMA pipe, for many threads hashing at once (the xors and rotations
 //    keep the ALU pipe busy);
-//  * ADD_MIXED: half of them, for one thread or warp hashing alone (the device channel, the
-//    FRI tail), whose time is the latency of its own chain. A chain of compressions by one
-//    warp takes 1477 cycles each, against 1640 with every addition on the ALU pipe (a + b + m
-//    as one) and 1960 with every one on the FMA pipe.
+//  * ADD_MIXED: half of them, for one thread or warp hashing alone (the FRI tail's levels),
+//    whose time is the latency of its own chain. B200, cycles a compression in a chain by one
+//    warp: 1665 when the message starts with the last digest and 1629 with a constant message;
+//    with every addition on the FMA pipe 1863 and 1725, with none there 1695 and 1653.
+// `one` has to be a run-time value for either: from a literal 1 the compiler makes plain
+// additions of both forms (the same 1695 and 1653). The channel's callers pass a literal, a
+// difference of 2% on two compressions a step.
 enum AddForm { ADD_FMA, ADD_MIXED };
 
 // a + b + m[S] (the first or second of a G's two) for a message whose words from W on are

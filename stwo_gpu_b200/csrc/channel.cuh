@@ -30,8 +30,8 @@ struct DevChannel {
 };
 
 // BLAKE2s-256 (RFC 7693, unkeyed, 32-byte digest) of the words word(0..n_words-1),
-// little endian. One thread runs the channel, so its compressions take the
-// short-chain form (ADD_MIXED).
+// little endian. One thread runs the channel, so its compressions keep off the long FMA
+// chain: with a literal 1 all their additions are plain ones (AddForm).
 template <class W>
 __device__ void blake2s_words(W word, uint32_t n_words, uint32_t out[8]) {
     const uint32_t one = 1;

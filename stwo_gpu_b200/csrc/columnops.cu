@@ -111,8 +111,10 @@ __global__ void __launch_bounds__(BI_THREADS) batch_inverse_m31_kernel(const uin
 // values are the same. Bound by instruction issue next to HBM (32 bytes an element): no
 // shuffle scans (as above), CM31 products as two-term dot products with one three-
 // instruction reduction (m31_dot2), and 72 registers for seven CTAs of 128 threads an SM.
-// 9999991 elements: 86.1 -> 65.5 us, 2^24: 139 -> 103 us (5.2 TB/s, 80% of the measured
-// copy rate); 6 elements a thread 65.6, 4: 71.6, 12: 68.5; CTAs of 256 threads 67.6-69.6.
+// Calls one after another, us: 9999991 elements 82.9 -> 67.8, 2^24 133 -> 95 (5.6 TB/s, 86%
+// of the measured copy rate); under the profiler 2^24 takes 139 -> 103. The kernel alone
+// on 9999991: 65.5 with 8 elements a thread, 65.6 with 6, 71.6 with 4, 68.5 with 12, and
+// 67.6-69.6 in CTAs of 256 threads.
 __global__ void __launch_bounds__(BI_THREADS, 7) batch_inverse_qm31_norm_kernel(const qm31 *__restrict__ src,
                                                                                 qm31 *__restrict__ dst, uint64_t n) {
     chain_wait();
@@ -209,8 +211,8 @@ int batch_inverse_m31_async(const uint32_t *src, uint32_t *dst, uint64_t n, cuda
 int batch_inverse_qm31_async(const uint32_t *src, uint32_t *dst, uint64_t n, cudaStream_t st) {
     if (n == 0) return STWO_OK;
     uint64_t blocks = (n + BI_THREADS * BI_QM31_PER_THREAD - 1) / (BI_THREADS * BI_QM31_PER_THREAD);
-    launch_chained(batch_inverse_qm31_norm_kernel, (unsigned)blocks, BI_THREADS, 0, st, reinterpret_cast<const qm31 *>(src),
-                                                                            reinterpret_cast<qm31 *>(dst), n);
+    launch_chained(batch_inverse_qm31_norm_kernel, (unsigned)blocks, BI_THREADS, 0, st,
+                   reinterpret_cast<const qm31 *>(src), reinterpret_cast<qm31 *>(dst), n);
     STWO_LAUNCH_CHECK("batch_inverse_qm31_norm_kernel");
     return STWO_OK;
 }

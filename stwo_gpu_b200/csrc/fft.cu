@@ -491,7 +491,8 @@ __device__ __forceinline__ void roundT(uint32_t *sm, const GeoT &geo) {
                         const uint32_t e = region + 4u * (i * 32u + lane);
                         const uint32_t *s2;
                         if (tile_column<G, C, T>(geo, e, s2, dst))
-                            t = __ldg(reinterpret_cast<const uint4 *>(s2 + (tile_index<G, C, LO, T>(geo, e) & p.src_mask)));
+                            t = __ldg(reinterpret_cast<const uint4 *>(
+                                s2 + (tile_index<G, C, LO, T>(geo, e) & p.src_mask)));
                     }
                     v[grp][4 * i] = t.x; v[grp][4 * i + 1] = t.y; v[grp][4 * i + 2] = t.z; v[grp][4 * i + 3] = t.w;
                 }
@@ -593,7 +594,8 @@ __device__ __forceinline__ void roundsT(uint32_t *sm, const GeoT &geo, std::inte
 // with 112-128 registers, and 2132 with four CTAs per SM (64 registers). 2^5 elements
 // a thread (512 threads): two CTAs per SM (64 registers; at three it spills).
 template <int G, int C, bool INV, int E, int LO, int T>
-__global__ void __launch_bounds__(1 << (T - E), E == 6 ? 3 : 2) fftT_kernel(const __grid_constant__ FftLaunch p, uint32_t n_cols) {
+__global__ void __launch_bounds__(1 << (T - E), E == 6 ? 3 : 2)
+    fftT_kernel(const __grid_constant__ FftLaunch p, uint32_t n_cols) {
     extern __shared__ __align__(16) uint32_t sm[];
     chain_wait();
     GeoT geo;
@@ -636,7 +638,8 @@ int launchT_e(const FftLaunch &p, uint32_t n_cols, cudaStream_t st) {
     if (rc) return rc;
     const uint64_t blocks = p.N >= (uint32_t)T ? (uint64_t)n_cols << (p.N - T)
                                                 : ((uint64_t)n_cols + (1u << (T - p.N)) - 1) >> (T - p.N);
-    STWO_REQUIRE(blocks < (1ull << 31), STWO_ERR_UNSUPPORTED_SIZE, "fft launch of %llu tiles", (unsigned long long)blocks);
+    STWO_REQUIRE(blocks < (1ull << 31), STWO_ERR_UNSUPPORTED_SIZE, "fft launch of %llu tiles",
+                 (unsigned long long)blocks);
     launch_chained(kern, (unsigned)blocks, 1 << (T - E), smem, st, p, n_cols);
     STWO_LAUNCH_CHECK("fftT_kernel");
     return STWO_OK;
@@ -646,9 +649,10 @@ int launchT_e(const FftLaunch &p, uint32_t n_cols, cudaStream_t st) {
 // threads per CTA) or 2^5 (512 threads): a tunable per pass kind and domain size
 // (stwo_autotune); 2^6 by default, measured faster at most sizes (us, strided passes with 2^6
 // and 2^5, both compiled for their row distance: interpolate 64 x 2^20 281 and 302, 8 x 2^22
-// 156 and 161, 8 x 2^24 672 and 693; evaluate 8 x 2^24 637 and 622). The tunables govern launches of more tiles than launchT_t spreads over more threads;
-// STWO_FFT_EPT_LOG (5 or 6) sets one value for all of them, the small ones too. Contiguous
-// passes of 4..10 layers always take 2^6, generic ones (launch_pass) neither.
+// 156 and 161, 8 x 2^24 672 and 693; evaluate 8 x 2^24 637 and 622). The tunables govern
+// launches of more tiles than launchT_t spreads over more threads; STWO_FFT_EPT_LOG (5 or
+// 6) sets one value for all of them, the small ones too. Contiguous passes of 4..10 layers
+// always take 2^6, generic ones (launch_pass) neither.
 inline int fft_ept_forced() {
     static const int forced = [] {
         const char *e = getenv("STWO_FFT_EPT_LOG");
@@ -960,7 +964,8 @@ int fft_columns_tab(const uint32_t *const *srcs, uint32_t *const *dsts, uint32_t
     const FftColumn *table = nullptr;
     void *staged = nullptr;
     if (n_cols > (uint32_t)MAX_COLS_PER_LAUNCH) {
-        const intptr_t src_step = (intptr_t)srcs[1] - (intptr_t)srcs[0], dst_step = (intptr_t)dsts[1] - (intptr_t)dsts[0];
+        const intptr_t src_step = (intptr_t)srcs[1] - (intptr_t)srcs[0];
+        const intptr_t dst_step = (intptr_t)dsts[1] - (intptr_t)dsts[0];
         bool equidistant = src_step > 0 && dst_step > 0 && src_step < (1ll << 34) && dst_step < (1ll << 34);
         for (uint32_t i = 1; i < n_cols && equidistant; i++)
             equidistant = (intptr_t)srcs[i] - (intptr_t)srcs[i - 1] == src_step &&

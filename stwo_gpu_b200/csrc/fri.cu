@@ -157,8 +157,11 @@ int fold_async(const uint32_t *const *src4, uint64_t n, stwo_qm31 alpha_c, const
             t[1] = m31_neg(iy);
         }
         if (circle)
-            launch_chained(fold_small_kernel<true>, jobs, 1, 0, st, s, d, (uint32_t)n_out, t[0], t[1], (const uint32_t *)nullptr, alpha, a2, ad, js);
-        else launch_chained(fold_small_kernel<false>, jobs, 1, 0, st, s, d, (uint32_t)n_out, 0u, 0u, tw, alpha, a2, ad, js);
+            launch_chained(fold_small_kernel<true>, jobs, 1, 0, st, s, d, (uint32_t)n_out, t[0], t[1],
+                           (const uint32_t *)nullptr, alpha, a2, ad, js);
+        else
+            launch_chained(fold_small_kernel<false>, jobs, 1, 0, st, s, d, (uint32_t)n_out, 0u, 0u, tw, alpha, a2, ad,
+                           js);
         STWO_LAUNCH_CHECK("fold_small_kernel");
         return STWO_OK;
     }
@@ -173,7 +176,8 @@ int fold_async(const uint32_t *const *src4, uint64_t n, stwo_qm31 alpha_c, const
         if (circle) launch_chained(fold_kernel<true, true>, grid, 256, 0, st, s, d, n_out, tw, alpha, a2, ad, js);
         else launch_chained(fold_kernel<false, true>, grid, 256, 0, st, s, d, n_out, tw, alpha, a2, ad, js);
     } else {
-        if (circle) launch_chained(fold_kernel<true, false>, grid, 256, 0, st, s, d, n_out, tw, alpha, a2, ad, (size_t)0);
+        if (circle)
+            launch_chained(fold_kernel<true, false>, grid, 256, 0, st, s, d, n_out, tw, alpha, a2, ad, (size_t)0);
         else launch_chained(fold_kernel<false, false>, grid, 256, 0, st, s, d, n_out, tw, alpha, a2, ad, (size_t)0);
     }
     STWO_LAUNCH_CHECK("fold_kernel");

@@ -103,9 +103,10 @@ __global__ void __launch_bounds__(256) merkle_layer_kernel(uint32_t log_size, co
 // ceiling (81% of the slots) where it is dense, so both the instructions and the number of
 // copies count. Layers of four columns (the QM31 columns of the composition and of FRI,
 // half of their trees' compressions) take a form without the 120 additions of zero words;
-// full and padded chunks share one copy (but see launch_tree). B200, us: 4 columns at each of 2^12..2^22 643 ->
-// 573, 4 x 2^22 427 -> 388, 4 x 2^20 145 -> 134, 101 x 2^18 (a padded chunk) 152 -> 137;
-// 64 x 2^22 897 -> 896. Further copies cost more than they save: a zero-state form for
+// full and padded chunks share one copy (but see launch_tree). B200, us, whole calls with
+// their staged tables: 4 columns at each of 2^12..2^22 639 -> 567, 4 x 2^22 427 -> 388, 4 x
+// 2^20 145 -> 134, 101 x 2^18 (a padded chunk) 152 -> 137, 17 x 2^20 202 -> 178, 64 x 2^22
+// 897 -> 896; 64..200 columns of 2^16 are 2-3% slower for it (55.6 -> 57.0 with 128). Further copies cost more than they save: a zero-state form for
 // leaves beside this one 412 at 4 x 2^22, an eight-word form 659 over the mixed tree; one
 // copy for children and chunks alike 929 at 64 x 2^22.
 constexpr int MERKLE_MAX_BANDS = 6;
@@ -319,8 +320,8 @@ void launch_tree(const TreeParams &p, uint32_t max_log, uint32_t blocks, uint32_
         inner += l < max_log && p.n_cols[l] != 0 && p.n_cols[l] != 4;
     }
     few = few && inner >= std::max(1, (int)max_log - 13);
-    launch_chained(few ? merkle_tree_kernel<THREADS, true> : merkle_tree_kernel<THREADS, false>, dim3(blocks, jobs), THREADS,
-                   0, st, p, 1u);
+    launch_chained(few ? merkle_tree_kernel<THREADS, true> : merkle_tree_kernel<THREADS, false>, dim3(blocks, jobs),
+                   THREADS, 0, st, p, 1u);
 }
 
 template <int CAP>
@@ -330,11 +331,12 @@ void launch_layer(uint32_t log_size, const uint32_t *prev, const uint32_t *const
     if (!cols_on_device)
         for (uint32_t i = 0; i < n_cols; i++) mc.c[i] = cols[i];
     if (cols_on_device)
-        launch_chained(merkle_layer_kernel<true, CAP>, blocks, 256, 0, st, log_size, reinterpret_cast<const uint4 *>(prev), mc,
-                                                               cols, n_cols, reinterpret_cast<uint4 *>(out), 1u);
+        launch_chained(merkle_layer_kernel<true, CAP>, blocks, 256, 0, st, log_size,
+                       reinterpret_cast<const uint4 *>(prev), mc, cols, n_cols, reinterpret_cast<uint4 *>(out), 1u);
     else
-        launch_chained(merkle_layer_kernel<false, CAP>, blocks, 256, 0, st, log_size, reinterpret_cast<const uint4 *>(prev), mc,
-                                                                (const uint32_t *const *)nullptr, n_cols, reinterpret_cast<uint4 *>(out), 1u);
+        launch_chained(merkle_layer_kernel<false, CAP>, blocks, 256, 0, st, log_size,
+                       reinterpret_cast<const uint4 *>(prev), mc, (const uint32_t *const *)nullptr, n_cols,
+                       reinterpret_cast<uint4 *>(out), 1u);
 }
 
 }  // namespace

@@ -663,7 +663,8 @@ int quotients_async(uint32_t half_init, uint32_t half_step, uint32_t log_size, c
         constexpr int NBV = decltype(nb)::value;
         using PR = std::decay_t<decltype(*holder)>;
         if (cols_on_device)
-            launch_chained(quotients_kernel<true, NBV, PR>, (unsigned)blocks, 256, smem, st, *holder, cols, n_stage, 2u);
+            launch_chained(quotients_kernel<true, NBV, PR>, (unsigned)blocks, 256, smem, st, *holder, cols, n_stage,
+                           2u);
         else
             launch_chained(quotients_kernel<false, NBV, PR>, (unsigned)blocks, 256, smem, st, *holder,
                            (const uint32_t *const *)nullptr, n_stage, 2u);

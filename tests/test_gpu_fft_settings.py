@@ -62,7 +62,8 @@ def run(shapes, tunables=(), env=None, autotune=False):
     spec = json.dumps({"shapes": shapes, "tunables": list(tunables), "autotune": autotune})
     e = {k: v for k, v in os.environ.items() if k != "STWO_FFT_EPT_LOG"}
     e.update(env or {})
-    r = subprocess.run([sys.executable, "-c", PROGRAM, spec], cwd=ROOT, env=e, capture_output=True, text=True, timeout=300)
+    r = subprocess.run([sys.executable, "-c", PROGRAM, spec], cwd=ROOT, env=e, capture_output=True, text=True,
+                       timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
     got = json.loads(r.stdout.strip().splitlines()[-1])
     if not got["passes"]:
@@ -74,8 +75,8 @@ def test_forced_elements_per_thread_reach_every_pass():
     """Small launches, which spread over more threads by themselves, and large ones."""
     shapes = [[1, 11, 1], [64, 12, 1], [3, 13, 2], [1, 14, 1], [4, 16, 1], [700, 12, 1]]
     base = run(shapes)
-    assert {(g, ept, t) for g, c, _, ept, _, t, _ in base["passes"] if c == 0} >= {(11, 4, 12), (12, 4, 12), (13, 5, 13),
-                                                                               (14, 5, 14)}
+    small = {(11, 4, 12), (12, 4, 12), (13, 5, 13), (14, 5, 14)}
+    assert {(g, ept, t) for g, c, _, ept, _, t, _ in base["passes"] if c == 0} >= small
     for value in (5, 6):
         got = run(shapes, env={"STWO_FFT_EPT_LOG": str(value)})
         assert {(ept, t) for *_, ept, _, t, _ in got["passes"]} == {(value, 14)}
