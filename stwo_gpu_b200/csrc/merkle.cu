@@ -106,9 +106,10 @@ __global__ void __launch_bounds__(256) merkle_layer_kernel(uint32_t log_size, co
 // full and padded chunks share one copy (but see launch_tree). B200, us, whole calls with
 // their staged tables: 4 columns at each of 2^12..2^22 639 -> 567, 4 x 2^22 427 -> 388, 4 x
 // 2^20 145 -> 134, 101 x 2^18 (a padded chunk) 152 -> 137, 17 x 2^20 202 -> 178, 64 x 2^22
-// 897 -> 896; 64..200 columns of 2^16 are 2-3% slower for it (55.6 -> 57.0 with 128). Further copies cost more than they save: a zero-state form for
-// leaves beside this one 412 at 4 x 2^22, an eight-word form 659 over the mixed tree; one
-// copy for children and chunks alike 929 at 64 x 2^22.
+// 897 -> 896; 64..200 columns of 2^16 are 2-3% slower for it (55.6 -> 57.0 with 128).
+// Further copies cost more than they save: a zero-state form for leaves beside this one 412
+// at 4 x 2^22, an eight-word form 659 at 4 columns of each of 2^12..2^22; one copy for
+// children and chunks alike 929 at 64 x 2^22.
 constexpr int MERKLE_MAX_BANDS = 6;
 
 struct TreeBand {
